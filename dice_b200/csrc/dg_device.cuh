@@ -91,6 +91,36 @@ struct DevGeometry {
 };
 
 // ---------------------------------------------------------------------------
+// Packed float pairs: two products or two sums per instruction, each rounded
+// on its own like the scalar ones.  The pipe takes the same time (35 Tera
+// operations a second either way), the issue slots halve.  ptxas contracts a
+// packed multiply and add into a fused one (not the reference's rounding), so
+// the product is written as a * b + (-0), which rounds like a * b with its
+// sign, and -0 comes as a run-time value (f2_minus_zero() as a kernel
+// argument), which keeps the compiler from simplifying it back.
+// ---------------------------------------------------------------------------
+typedef unsigned long long f32x2;
+__host__ __device__ constexpr f32x2 f2_minus_zero() { return 0x8000000080000000ull; }
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b, f32x2 minus_zero) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(minus_zero));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// ---------------------------------------------------------------------------
 // Warp reductions
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {

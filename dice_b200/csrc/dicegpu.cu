@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "dg_frame.cuh"
+#include "dg_image.cuh"
 #include "dg_adjoint.cuh"
 #include "dg_raster.cuh"
 #include "dg_vsg.cuh"
@@ -33,106 +34,6 @@ using namespace dg;
 #ifndef DG_QUEUE_CHUNK
 #define DG_QUEUE_CHUNK 0
 #endif
-
-// ---------------------------------------------------------------------------
-// gradients
-// ---------------------------------------------------------------------------
-// Finite differences with c1 = 1/12, c2 = -8/12 stored as float
-// (DICe_Image.cpp:214-215), one-sided within two pixels of the border.
-// Separate rounded products and sums (no contraction) so that the result is
-// bit-identical to the reference's expression order.
-__global__ void gradient_fd_kernel(int w, int h, const float* __restrict__ I, float* __restrict__ gx,
-                                   float* __restrict__ gy) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y;
-  if (x >= w || y >= h) return;
-  const float c1 = (float)(1.0 / 12.0), c2 = (float)(-8.0 / 12.0);
-  const size_t i = (size_t)y * w + x;
-  float a, b;
-  if (x < 2) a = __fsub_rn(I[i + 1], I[i]);
-  else if (x >= w - 2) a = __fsub_rn(I[i], I[i - 1]);
-  else a = __fsub_rn(__fsub_rn(__fadd_rn(__fmul_rn(c1, I[i - 2]), __fmul_rn(c2, I[i - 1])),
-                               __fmul_rn(c2, I[i + 1])),
-                     __fmul_rn(c1, I[i + 2]));
-  if (y < 2) b = __fsub_rn(I[i + w], I[i]);
-  else if (y >= h - 2) b = __fsub_rn(I[i], I[i - w]);
-  else b = __fsub_rn(__fsub_rn(__fadd_rn(__fmul_rn(c1, I[i - 2 * (size_t)w]), __fmul_rn(c2, I[i - w])),
-                               __fmul_rn(c2, I[i + w])),
-                     __fmul_rn(c1, I[i + 2 * (size_t)w]));
-  gx[i] = a;
-  gy[i] = b;
-}
-
-// smooth_gradients_convolution_5_point (DICe_Image.cpp:1034-1060): outer
-// product of (1,4,6,4,1)/16 on the interior, borders copied.
-__global__ void gradient_smooth_kernel(int w, int h, const float* __restrict__ tx,
-                                       const float* __restrict__ ty, float* __restrict__ gx,
-                                       float* __restrict__ gy) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y;
-  if (x >= w || y >= h) return;
-  const size_t i = (size_t)y * w + x;
-  if (x < 2 || x >= w - 2 || y < 2 || y >= h - 2) {
-    gx[i] = tx[i];
-    gy[i] = ty[i];
-    return;
-  }
-  const float k[5] = {0.0625f, 0.25f, 0.375f, 0.25f, 0.0625f};
-  float vx = 0.0f, vy = 0.0f;
-#pragma unroll
-  for (int a = 0; a < 5; ++a)
-#pragma unroll
-    for (int b = 0; b < 5; ++b) {
-      const float c = __fmul_rn(k[a], k[b]);
-      const size_t j = (size_t)(y + a - 2) * w + x + b - 2;
-      vx = __fadd_rn(vx, __fmul_rn(c, tx[j]));
-      vy = __fadd_rn(vy, __fmul_rn(c, ty[j]));
-    }
-  gx[i] = vx;
-  gy[i] = vy;
-}
-
-// Image_::gauss_filter (DICe_Image.cpp:1194-1230).  The M x M weights travel
-// by value in the parameter bank (uniform reads); each CTA stages its
-// (32 + M - 1) x (8 + M - 1) input tile in shared memory.  The sum runs x
-// offset outer, y offset inner, with every float product and sum rounded
-// separately, as the reference's loop does; pixels within M/2+1 of an edge
-// keep their value.
-struct GaussWeights {
-  float c[13 * 13];
-};
-
-constexpr int kGaussBX = 32, kGaussBY = 8, kGaussMaxTile = (kGaussBX + 12) * (kGaussBY + 12);
-
-__global__ void __launch_bounds__(kGaussBX * kGaussBY)
-gauss_filter_kernel(int w, int h, int M, const GaussWeights wt, const float* __restrict__ in,
-                    float* __restrict__ out) {
-  __shared__ float tile[kGaussMaxTile];
-  const int R = M / 2;                 // taps reach R pixels either side
-  const int half = M / 2 + 1;          // the reference's interior test
-  const int TW = kGaussBX + 2 * R, TH = kGaussBY + 2 * R;
-  const int x0 = blockIdx.x * kGaussBX - R, y0 = blockIdx.y * kGaussBY - R;
-  const int tid = threadIdx.y * kGaussBX + threadIdx.x;
-  for (int k = tid; k < TW * TH; k += kGaussBX * kGaussBY) {
-    const int ty = k / TW, tx = k - ty * TW;
-    const int gx = x0 + tx, gy = y0 + ty;
-    tile[k] = (gx >= 0 && gx < w && gy >= 0 && gy < h) ? in[(size_t)gy * w + gx] : 0.0f;
-  }
-  __syncthreads();
-  const int x = blockIdx.x * kGaussBX + threadIdx.x;
-  const int y = blockIdx.y * kGaussBY + threadIdx.y;
-  if (x >= w || y >= h) return;
-  const size_t o = (size_t)y * w + x;
-  if (!(x >= half && x < w - half && y >= half && y < h - half)) {
-    out[o] = in[o];
-    return;
-  }
-  float v = 0.0f;
-  for (int i = 0; i < M; ++i)
-    for (int j = 0; j < M; ++j)
-      v = __fadd_rn(v, __fmul_rn(wt.c[i * M + j], tile[(threadIdx.y + j) * TW + threadIdx.x + i]));
-  out[o] = v;
-}
 
 // Incremental formulation (DICe_Schema.cpp:1671-1675, 1775-1789): a frame
 // after the first starts with DISPLACEMENT_X / _Y at 0 and ends with them
@@ -158,13 +59,6 @@ __global__ void incr_end_kernel(double* __restrict__ fields, double* __restrict_
 __global__ void evo_rebase_kernel(uint8_t* __restrict__ state, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && state[i] == 2) state[i] = 1;
-}
-
-// (I, Gx, Gy) -> interleaved float4 (the layout the frame kernel gathers from)
-__global__ void pack_kernel(size_t n, const float* __restrict__ I, const float* __restrict__ gx,
-                            const float* __restrict__ gy, float4* __restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = make_float4(I[i], gx[i], gy[i], 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -271,7 +165,7 @@ struct dicegpu_ctx {
   float* d_def = nullptr;
   float* d_def_gx = nullptr;
   float* d_def_gy = nullptr;
-  float* d_tmp = nullptr;   // smoothing scratch (2 planes)
+  float* d_tmp = nullptr;   // upload staging (2 planes)
   float4* d_def4 = nullptr; // deformed (I, Gx, Gy, 0) interleaved
   size_t img_cap = 0;       // pixels allocated per plane
   bool has_ref = false, has_def = false;
@@ -622,50 +516,59 @@ static int ensure_images(dicegpu_ctx* c, int w, int h) {
   return DICEGPU_OK;
 }
 
-static int launch_gradients(int w, int h, const float* img, float* gx, float* gy, int method,
-                            float* tmp, cudaStream_t st, long long* launches) {
-  dim3 blk(256), grd((w + 255) / 256, h);
+// a float twice, as the packed operations take it
+static f32x2 pair_of(float v) {
+  uint32_t b;
+  std::memcpy(&b, &v, 4);
+  return ((f32x2)b << 32) | b;
+}
+
+static int launch_gradients(int w, int h, const float* img, float* gx, float* gy, int method, cudaStream_t st,
+                            long long* launches) {
   if (method == DICEGPU_CONVOLUTION_5_POINT) {
-    float* tx = tmp;
-    float* ty = tmp + (size_t)w * h;
-    gradient_fd_kernel<<<grd, blk, 0, st>>>(w, h, img, tx, ty);
-    gradient_smooth_kernel<<<grd, blk, 0, st>>>(w, h, tx, ty, gx, gy);
-    if (launches) *launches += 2;
+    const dim3 blk(kSmoothB, kSmoothBY), grd((w + kSmoothB - 1) / kSmoothB, (h + kSmoothB - 1) / kSmoothB);
+    SmoothWeights wt;
+    const float k5[3] = {0.0625f, 0.25f, 0.375f};
+    for (int a = 0; a < 3; ++a)
+      for (int b = 0; b < 3; ++b) wt.k[a][b] = pair_of(k5[a] * k5[b]);
+    gradient_smooth_kernel<<<grd, blk, 0, st>>>(w, h, wt, f2_minus_zero(), img, gx, gy);
   } else {
+    const dim3 blk(256), grd((w + 255) / 256, h);
     gradient_fd_kernel<<<grd, blk, 0, st>>>(w, h, img, gx, gy);
-    if (launches) *launches += 1;
   }
   CK(cudaGetLastError());
+  if (launches) *launches += 1;
   return DICEGPU_OK;
 }
 
 // The reference's Gaussian masks are outer products of these 1-D weights
 // with every product printed to 9 significant digits (DICe_Image.cpp:54-112);
-// rounding the same way gives the identical float tables.
+// rounding the same way gives the identical float tables.  The five tables
+// are made once (printing and reading 49 numbers takes 25 us, more than the
+// kernel at 512^2).
 static bool gauss_weights(int M, GaussWeights& g) {
-  static const double w5[] = {0.0014, 0.1574, 0.62825};
-  static const double w7[] = {0.006, 0.0606, 0.2418, 0.3831};
-  static const double w9[] = {0.0007, 0.0108, 0.0748, 0.2384, 0.3505};
-  static const double w11[] = {0.0001, 0.0017, 0.0168, 0.087, 0.2328, 0.3231};
-  static const double w13[] = {0.0001, 0.0012, 0.0085, 0.038, 0.1109, 0.2108, 0.2611};
-  const double* half;
-  switch (M) {
-    case 5: half = w5; break;
-    case 7: half = w7; break;
-    case 9: half = w9; break;
-    case 11: half = w11; break;
-    case 13: half = w13; break;
-    default: return false;
-  }
-  const int R = M / 2;
-  double w[13];
-  for (int i = 0; i < M; ++i) w[i] = half[i <= R ? i : M - 1 - i];
-  for (int i = 0; i < M; ++i)
-    for (int j = 0; j < M; ++j) {
-      char buf[32];
-      std::snprintf(buf, sizeof(buf), "%.8e", w[i] * w[j]);
-      g.c[i * M + j] = (float)std::strtod(buf, nullptr);
+  if (M < 5 || M > 13 || !(M & 1)) return false;
+  static const std::vector<GaussWeights> tables = [] {
+    static const double half[5][7] = {{0.0014, 0.1574, 0.62825},
+                                      {0.006, 0.0606, 0.2418, 0.3831},
+                                      {0.0007, 0.0108, 0.0748, 0.2384, 0.3505},
+                                      {0.0001, 0.0017, 0.0168, 0.087, 0.2328, 0.3231},
+                                      {0.0001, 0.0012, 0.0085, 0.038, 0.1109, 0.2108, 0.2611}};
+    std::vector<GaussWeights> all(5);
+    for (int k = 0; k < 5; ++k) {
+      const int m = 5 + 2 * k, R = m / 2;
+      double w[13];
+      for (int i = 0; i < m; ++i) w[i] = half[k][i <= R ? i : m - 1 - i];
+      for (int i = 0; i < m; ++i)
+        for (int j = 0; j < m; ++j) {
+          char buf[32];
+          std::snprintf(buf, sizeof(buf), "%.8e", w[i] * w[j]);
+          all[k].c[i * m + j] = pair_of((float)std::strtod(buf, nullptr));
+        }
     }
+    return all;
+  }();
+  g = tables[(M - 5) / 2];
   return true;
 }
 
@@ -674,8 +577,20 @@ static int launch_gauss_filter(int w, int h, int M, const float* in, float* out,
   GaussWeights g;
   if (!gauss_weights(M, g)) return DICEGPU_ERR_ARG;
   if (w < M || h < M) return DICEGPU_ERR_ARG;
-  dim3 blk(kGaussBX, kGaussBY), grd((w + kGaussBX - 1) / kGaussBX, (h + kGaussBY - 1) / kGaussBY);
-  gauss_filter_kernel<<<grd, blk, 0, st>>>(w, h, M, g, in, out);
+  // eight rows a thread while that leaves every SM two CTAs, else two
+  const unsigned gx = (w + 2 * kGaussBX - 1) / (2 * kGaussBX);
+  const bool tall = (long long)gx * ((h + 8 * kGaussBY - 1) / (8 * kGaussBY)) >= 2 * 148;
+  const unsigned rows = kGaussBY * (tall ? 8 : 2);
+  const dim3 blk(kGaussBX, kGaussBY), grd(gx, (h + rows - 1) / rows);
+  void (*fn)(int, int, GaussWeights, f32x2, const float*, float*) = nullptr;
+  switch (M) {
+    case 5: fn = tall ? gauss_filter_kernel<5, 8> : gauss_filter_kernel<5, 2>; break;
+    case 7: fn = tall ? gauss_filter_kernel<7, 8> : gauss_filter_kernel<7, 2>; break;
+    case 9: fn = tall ? gauss_filter_kernel<9, 8> : gauss_filter_kernel<9, 2>; break;
+    case 11: fn = tall ? gauss_filter_kernel<11, 8> : gauss_filter_kernel<11, 2>; break;
+    default: fn = tall ? gauss_filter_kernel<13, 8> : gauss_filter_kernel<13, 2>; break;
+  }
+  fn<<<grd, blk, 0, st>>>(w, h, g, f2_minus_zero(), in, out);
   CK(cudaGetLastError());
   if (launches) *launches += 1;
   return DICEGPU_OK;
@@ -739,8 +654,8 @@ static int set_ref(dicegpu_ctx* c, int w, int h, const void* pixels, int type, i
   int rc = ensure_images(c, w, h);
   if (rc) return rc;
   if ((rc = upload_typed(c, c->d_ref, pixels, type, on_device))) return rc;
-  if ((rc = launch_gradients(w, h, c->d_ref, c->d_ref_gx, c->d_ref_gy, c->params.gradient_method,
-                             c->d_tmp, c->stream, &c->launches)))
+  if ((rc = launch_gradients(w, h, c->d_ref, c->d_ref_gx, c->d_ref_gy, c->params.gradient_method, c->stream,
+                             &c->launches)))
     return rc;
   c->has_ref = true;
   return DICEGPU_OK;
@@ -754,11 +669,11 @@ static int set_def(dicegpu_ctx* c, int w, int h, const void* pixels, int type, i
   if ((rc = upload_typed(c, c->d_def, pixels, type, on_device))) return rc;
   if (c->params.use_def_gradients) {
     if ((rc = launch_gradients(w, h, c->d_def, c->d_def_gx, c->d_def_gy, c->params.gradient_method,
-                               c->d_tmp, c->stream, &c->launches)))
+                               c->stream, &c->launches)))
       return rc;
     const size_t npx = (size_t)w * h;
-    pack_kernel<<<(unsigned)((npx + 255) / 256), 256, 0, c->stream>>>(npx, c->d_def, c->d_def_gx,
-                                                                      c->d_def_gy, c->d_def4);
+    pack_kernel<<<(unsigned)((npx + 255) / 256), 256, 0, c->stream>>>(npx, c->d_def, c->d_def_gx, c->d_def_gy,
+                                                                      c->d_def4);
     CK(cudaGetLastError());
     c->launches += 1;
   }
@@ -804,7 +719,7 @@ extern "C" int dicegpu_set_ref_from_def(dicegpu_ctx* c) {
   if (!c) return DICEGPU_ERR_ARG;
   if (!c->has_ref || !c->has_def) return DICEGPU_ERR_STATE;
   CK(cudaMemcpyAsync(c->d_ref, c->d_def, (size_t)c->W * c->H * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
-  return launch_gradients(c->W, c->H, c->d_ref, c->d_ref_gx, c->d_ref_gy, c->params.gradient_method, c->d_tmp,
+  return launch_gradients(c->W, c->H, c->d_ref, c->d_ref_gx, c->d_ref_gy, c->params.gradient_method,
                           c->stream, &c->launches);
 }
 
@@ -2326,19 +2241,28 @@ extern "C" int dicegpu_interpolate(dicegpu_ctx* c, int method, int n, const floa
   return rc;
 }
 
+// Whether the smoothing writes over its own input: a CTA reads pixels that
+// others have written by then, so the input is copied first.
+static bool smooth_in_place(int w, int h, const float* img, const float* gx, const float* gy, int method) {
+  const uintptr_t n = (uintptr_t)w * h * sizeof(float), a = (uintptr_t)img;
+  auto meets = [&](const float* p) { return (uintptr_t)p < a + n && a < (uintptr_t)p + n; };
+  return method == DICEGPU_CONVOLUTION_5_POINT && (meets(gx) || meets(gy));
+}
+
 extern "C" int dicegpu_image_gradients(int w, int h, const float* d_img, float* d_gx, float* d_gy,
                                        int method, void* stream) {
   if (!d_img || !d_gx || !d_gy || w < 3 || h < 3) return DICEGPU_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
+  if (!smooth_in_place(w, h, d_img, d_gx, d_gy, method))
+    return launch_gradients(w, h, d_img, d_gx, d_gy, method, st, nullptr);
+  const size_t bytes = (size_t)w * h * sizeof(float);
   float* tmp = nullptr;
-  if (method == DICEGPU_CONVOLUTION_5_POINT) {
-    if (cudaMalloc(&tmp, 2 * (size_t)w * h * sizeof(float)) != cudaSuccess) return DICEGPU_ERR_NOMEM;
-  }
-  int rc = launch_gradients(w, h, d_img, d_gx, d_gy, method, tmp, st, nullptr);
-  if (tmp) {
-    cudaStreamSynchronize(st);
-    cudaFree(tmp);
-  }
+  if (cudaMalloc(&tmp, bytes) != cudaSuccess) return DICEGPU_ERR_NOMEM;
+  int rc = cudaMemcpyAsync(tmp, d_img, bytes, cudaMemcpyDeviceToDevice, st) == cudaSuccess ? DICEGPU_OK
+                                                                                         : DICEGPU_ERR_CUDA;
+  if (rc == DICEGPU_OK) rc = launch_gradients(w, h, tmp, d_gx, d_gy, method, st, nullptr);
+  cudaStreamSynchronize(st);
+  cudaFree(tmp);
   return rc;
 }
 
@@ -2354,10 +2278,10 @@ extern "C" int dicegpu_gauss_filter(int w, int h, const float* d_in, float* d_ou
 // For callers that cannot allocate device memory themselves: hosts that give
 // the library a fixed device-memory budget owned by their own pool, or
 // per-frame loops that cannot afford cudaMalloc / cudaFree (cudaFree waits
-// for the whole device).  The two intermediate finite-difference planes that
-// dicegpu_image_gradients allocates for the 5-point smoothing live instead in
-// the file-scope array below, which every GPU that loads this library holds
-// until the process exits (8 MiB).
+// for the whole device).  The copy that dicegpu_image_gradients allocates
+// when the 5-point smoothing writes over its own input lives instead in the
+// file-scope array below, which every GPU that loads this library holds until
+// the process exits (8 MiB).
 // ---------------------------------------------------------------------------
 static __device__ __align__(256) float g_noalloc_scratch[2 * DICEGPU_NOALLOC_MAX_PIXELS];
 
@@ -2388,16 +2312,15 @@ extern "C" int dicegpu_image_gradients_noalloc(int w, int h, const float* d_img,
   if (!d_img || !d_gx || !d_gy || w < 3 || h < 3) return DICEGPU_ERR_ARG;
   if (method != DICEGPU_FINITE_DIFFERENCE && method != DICEGPU_CONVOLUTION_5_POINT)
     return DICEGPU_ERR_ARG;
-  float* tmp = nullptr;
-  if (method == DICEGPU_CONVOLUTION_5_POINT) {
-    // only the smoothing step needs the intermediate planes
-    if ((long long)w * h > DICEGPU_NOALLOC_MAX_PIXELS) return DICEGPU_ERR_ARG;
+  if (method == DICEGPU_CONVOLUTION_5_POINT && (long long)w * h > DICEGPU_NOALLOC_MAX_PIXELS) return DICEGPU_ERR_ARG;
+  if (smooth_in_place(w, h, d_img, d_gx, d_gy, method)) {
+    float* tmp = nullptr;
     const int rc = noalloc_scratch(&tmp);
     if (rc) return rc;
+    CK(cudaMemcpyAsync(tmp, d_img, (size_t)w * h * sizeof(float), cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
+    d_img = tmp;
   }
-  // the finite-difference kernel writes every scratch element the smoothing
-  // kernel reads, so nothing needs clearing between calls
-  return launch_gradients(w, h, d_img, d_gx, d_gy, method, tmp, (cudaStream_t)stream, nullptr);
+  return launch_gradients(w, h, d_img, d_gx, d_gy, method, (cudaStream_t)stream, nullptr);
 }
 
 // dice_correlate's stride-9 interface (DICe_api.cpp:51-151).  As the
