@@ -2,7 +2,7 @@
 //
 // frame_kernel<shape, interp, defgrad, mask> runs Schema::execute_correlation
 // (or one Objective entry point, by mode) for every subset of a launch: one
-// CTA per subset from interleaved per-CTA work queues.  The instantiations
+// CTA per subset, handed out in order.  The instantiations
 // live in frame_inst.cu (one unit per shape function, interpolation and
 // mask); the unmasked kernels are exactly what they are without masks.
 #pragma once
@@ -34,43 +34,30 @@ __global__ void __launch_bounds__(DG_MAX_THREADS, DG_MIN_BLOCKS) frame_kernel(co
   }
   // the launch's subsets: all n, or the n_order listed in order
   const int count = a.order ? a.n_order : a.n;
-  if (a.queue_mode == 0) {
-    // one global queue head
-    for (;;) {
-      if (threadIdx.x == 0) c.work = atomicAdd(a.work_counter, 1);
-      __syncthreads();
-      const int t = c.work;
-      __syncthreads();
-      if (t >= count) break;
-      e.run(a.order ? a.order[t] : t);
-    }
-    return;
-  }
-  // Interleaved per-CTA queues: the subsets are cut into chunks of C
-  // consecutive ones and CTA r owns chunks r, r + G, r + 2G, ...  All CTAs
-  // advance through the image together (a narrow band resident in L2).  A
-  // CTA whose chunks are exhausted takes from the following CTAs' sequences.
-  // Every index is taken exactly once (atomicAdd); a CTA leaves after finding
-  // all G sequences exhausted, so no CTA ever waits on another.
-  const int G = gridDim.x;
+  // The launch's chunks of C consecutive subsets are handed out in order: the
+  // first gridDim.x to the CTAs by number, the others from one counter, so that
+  // all CTAs advance through the image together (a narrow band resident in
+  // L2) and a CTA that finds the counter past the end is done.  Every chunk
+  // is taken exactly once and no CTA ever waits on another.  (With a queue
+  // per CTA and stealing, a CTA had to find every one of the 296 or 592
+  // queues empty before it could leave: about 90 us at the end of every
+  // launch, most of a tracking wave's time.)
   const int C = a.chunk;
-  int q = blockIdx.x;
-  for (int visited = 0; visited < G;) {
-    if (threadIdx.x == 0) c.work = atomicAdd(a.work_counter + q, 1);
-    __syncthreads();
-    const int t = c.work;
-    __syncthreads();
-    const long long chunk = (long long)q + (long long)(t / C) * G;
-    const long long lidx = chunk * C + (t % C);
-    const int pos = lidx < count ? (int)lidx : count;
-    if (pos < count) {
+  const int chunks = (count + C - 1) / C;
+  for (int t = blockIdx.x; t < chunks;) {
+    const int end = min((t + 1) * C, count);
+#pragma unroll 1
+    for (int pos = t * C; pos < end; ++pos) {
       DG_PT(t_run);
       e.run(a.order ? a.order[pos] : pos);
       DG_PACC(0, t_run);
-      continue;
+      __syncthreads();
     }
-    ++visited;
-    q = (q + 1 == G) ? 0 : q + 1;
+    if (chunks <= gridDim.x) return;
+    if (threadIdx.x == 0) c.work = gridDim.x + atomicAdd(a.work_counter, 1);
+    __syncthreads();
+    t = c.work;
+    __syncthreads();
   }
 }
 

@@ -30,11 +30,6 @@
 
 using namespace dg;
 
-// consecutive subsets per work-queue chunk (0: two per warp of a CTA)
-#ifndef DG_QUEUE_CHUNK
-#define DG_QUEUE_CHUNK 0
-#endif
-
 // Incremental formulation (DICe_Schema.cpp:1671-1675, 1775-1789): a frame
 // after the first starts with DISPLACEMENT_X / _Y at 0 and ends with them
 // set to the accumulated displacement.
@@ -132,8 +127,8 @@ __global__ void interp_kernel(int method, int w, int h, const float* __restrict_
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
-// upper bound on the persistent grid (and on its per-CTA queue heads)
-static const int kMaxQueues = 8192;
+// upper bound on the persistent grid
+static const int kMaxGrid = 8192;
 
 template <typename T>
 static int grow(T** p, size_t* cap, size_t need);
@@ -196,9 +191,7 @@ struct dicegpu_ctx {
   const void* wide_fn = nullptr;
   size_t wide_smem = 0;
   int wide_per_sm = 0;
-  int queue_mode = 1;    // 1: per-CTA queues with stealing, 0: one global queue
   int carveout = -1;     // preferred shared-memory carveout (percent), -1: driver default
-  int chunk = DG_QUEUE_CHUNK;   // queue chunk (consecutive subsets); 0: 2 per warp of a CTA
   long long launches = 0;
   // captured frame sequence
   cudaStream_t cap_stream = nullptr;
@@ -410,7 +403,7 @@ extern "C" int dicegpu_create(const dicegpu_params* params, dicegpu_ctx** out) {
   if (cudaGetDevice(&c->device) != cudaSuccess ||
       cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
       cudaDeviceGetAttribute(&c->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess ||
-      cudaMalloc(&c->d_counter, kMaxQueues * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&c->d_counter, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess ||
       cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess) {
     if (c->d_counter) cudaFree(c->d_counter);
@@ -1487,8 +1480,7 @@ static void fill_args(dicegpu_ctx* c, FrameArgs& a, int mode) {
   a.mode = mode;
   a.plain_index = -1;
   a.work_counter = c->d_counter;
-  a.queue_mode = c->queue_mode;
-  a.chunk = c->chunk > 0 ? c->chunk : 4;
+  a.chunk = 1;
   a.status = c->d_status;
   a.passes_out = c->d_passes;
   a.unc = (c->params.compute_uncertainty && c->unc_n == c->n) ? c->d_unc : nullptr;
@@ -1512,11 +1504,24 @@ static int grid_for(dicegpu_ctx* c, FrameKernelFn fn, int* blocks, size_t* smem)
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, threads, *smem));
     if (per_sm < 1) per_sm = 1;
   }
-  *blocks = std::min(per_sm * c->num_sms, kMaxQueues);
+  *blocks = std::min(per_sm * c->num_sms, kMaxGrid);
   if (c->pix_in_global) {
     int rc = c->d_pix_scratch.ensure((size_t)*blocks * pix);
     if (rc) return rc;
   }
+  return DICEGPU_OK;
+}
+
+// One launch of the frame kernel over the args' subsets (`count` of them): no
+// more CTAs than there are chunks; the counter is needed beyond one chunk each.
+static int launch_frame(dicegpu_ctx* c, FrameKernelFn fn, const FrameArgs& a, int count, int blocks, int warps,
+                        size_t smem) {
+  const int chunks = (count + a.chunk - 1) / a.chunk;
+  blocks = std::min(blocks, chunks);
+  if (chunks > blocks) CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
+  fn<<<blocks, warps * 32, smem, c->stream>>>(a);
+  CK(cudaGetLastError());
+  c->launches += 1;
   return DICEGPU_OK;
 }
 
@@ -1689,7 +1694,7 @@ static void wide_launch(dicegpu_ctx* c, FrameKernelFn fn, long n, int* warps, in
   const int per_sm = c->wide_per_sm;
   if (per_sm < 1) return;
   *warps = w;
-  *blocks = std::min(std::min(per_sm * c->num_sms, kMaxQueues), *blocks);
+  *blocks = std::min(std::min(per_sm * c->num_sms, kMaxGrid), *blocks);
   *smem = s;
 }
 
@@ -1741,14 +1746,10 @@ static int run_waves(dicegpu_ctx* c, int kind, FrameKernelFn fn, int blocks, siz
         ++L1;
       a.order = pl.d_wave.p + pl.wave_off[L];
       a.n_order = pl.wave_off[L1] - pl.wave_off[L];
-      a.queue_mode = 0;
       int cw = c->warps_per_cta;
       size_t csmem = smem;
       chain_shape(c, fn, &cw, &csmem);
-      CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
-      fn<<<1, cw * 32, csmem, c->stream>>>(a);
-      CK(cudaGetLastError());
-      c->launches += 1;
+      if ((rc = launch_frame(c, fn, a, a.n_order, 1, cw, csmem))) return rc;
       L = L1;
       continue;
     }
@@ -1767,10 +1768,7 @@ static int run_waves(dicegpu_ctx* c, int kind, FrameKernelFn fn, int blocks, siz
       int ww = c->warps_per_cta, wb = blocks;
       size_t ws = smem;
       wide_launch(c, fn, nw, &ww, &wb, &ws);
-      CK(cudaMemsetAsync(c->d_counter, 0, (size_t)wb * sizeof(int), c->stream));
-      fn<<<wb, ww * 32, ws, c->stream>>>(a);
-      CK(cudaGetLastError());
-      c->launches += 1;
+      if ((rc = launch_frame(c, fn, a, nw, wb, ww, ws))) return rc;
     }
     ++L;
   }
@@ -1794,10 +1792,7 @@ extern "C" int dicegpu_execute_correlation(dicegpu_ctx* c) {
   fill_args(c, a, MODE_CORRELATE);
   int warps = c->warps_per_cta;
   wide_launch(c, fn, c->n, &warps, &blocks, &smem);
-  CK(cudaMemsetAsync(c->d_counter, 0, (size_t)blocks * sizeof(int), c->stream));
-  fn<<<blocks, warps * 32, smem, c->stream>>>(a);
-  CK(cudaGetLastError());
-  c->launches += 1;
+  if ((rc = launch_frame(c, fn, a, c->n, blocks, warps, smem))) return rc;
   return frame_end(c);
 }
 
@@ -2072,10 +2067,8 @@ extern "C" int dicegpu_gamma(dicegpu_ctx* c, const double* fields, double* gamma
     a.fields = d_f;
     a.gamma_out = d_g;
     a.passes_out = nullptr;
-    if (cudaMemsetAsync(c->d_counter, 0, (size_t)blocks * sizeof(int), c->stream) != cudaSuccess) rc = DICEGPU_ERR_CUDA;
-    fn<<<blocks, c->warps_per_cta * 32, smem, c->stream>>>(a);
-    if (cudaGetLastError() != cudaSuccess) rc = DICEGPU_ERR_CUDA;
-    c->launches += 1;
+    const int rl = launch_frame(c, fn, a, c->n, blocks, c->warps_per_cta, smem);
+    if (!rc) rc = rl;
     if (!rc && cudaMemcpyAsync(gamma_out, d_g, c->n * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
       rc = DICEGPU_ERR_CUDA;
     if (!rc && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = DICEGPU_ERR_CUDA;
@@ -2121,11 +2114,8 @@ static int run_objective_mode(dicegpu_ctx* c, int mode, double* fields, int32_t*
     a.status_out = d_st;
     a.gamma_out = d_sg;
     a.noise_out = d_no;
-    if (cudaMemsetAsync(c->d_counter, 0, (size_t)blocks * sizeof(int), c->stream) != cudaSuccess)
-      rc = DICEGPU_ERR_CUDA;
-    fn<<<blocks, c->warps_per_cta * 32, smem, c->stream>>>(a);
-    if (cudaGetLastError() != cudaSuccess) rc = DICEGPU_ERR_CUDA;
-    c->launches += 1;
+    const int rl = launch_frame(c, fn, a, c->n, blocks, c->warps_per_cta, smem);
+    if (!rc) rc = rl;
   }
   auto d2h = [&](void* dst, const void* src, size_t b) {
     if (!rc && dst && cudaMemcpyAsync(dst, src, b, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
