@@ -28,6 +28,7 @@ struct DevParams {
   int N;           // number of parameters of the reference shape function
   int NS;          // number of slots (6 affine, 12 quadratic)
   int slot[12];
+  int cidx[12];    // compact index of each slot (-1: disabled)
   int has_rot;
   int interp;
   int opt;
@@ -272,6 +273,41 @@ __device__ __forceinline__ void keys_ref_interior(const DevImage& im, float x, f
   }
   iv = a;
   gxv = b;
+  gyv = c;
+}
+
+// The same value and gradients in a loop over row pairs, whose code a
+// scheduler's instruction cache holds (unrolled, the 36 taps are 5 KB, and
+// warps at different places of it wait for instructions), with the sums of I
+// and Gx as a packed pair.
+__device__ __forceinline__ void keys_ref_rows(const DevImage& im, float x, float y, float& iv, float& gxv,
+                                              float& gyv) {
+  const int ix = (int)x, iy = (int)y;
+  float wx[6], wy[6];
+  keys_weights_ref_interior(__fsub_rn(x, (float)ix), wx);
+  keys_weights_ref_interior(__fsub_rn(y, (float)iy), wy);
+  f32x2 ab = f2_pack(0.0f, 0.0f);
+  float c = 0.0f;
+  const float4* q = im.p4 + (size_t)(iy - 2) * im.w + (ix - 2);
+#pragma unroll 1
+  for (int m = 0; m < 3; ++m) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int n = 0; n < 6; ++n) {
+        const float4 t = __ldg(q + n);
+        const float cc = __fmul_rn(wy[h], wx[n]);
+        ab = f2_add(ab, f2_pack(__fmul_rn(cc, t.x), __fmul_rn(cc, t.y)));
+        c = __fadd_rn(c, __fmul_rn(cc, t.z));
+      }
+      q += im.w;
+    }
+    wy[0] = wy[2];
+    wy[1] = wy[3];
+    wy[2] = wy[4];
+    wy[3] = wy[5];
+  }
+  f2_unpack(ab, iv, gxv);
   gyv = c;
 }
 

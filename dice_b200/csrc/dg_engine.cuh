@@ -359,14 +359,21 @@ struct Engine {
     Ctl& c = ctl();
     const WarpOut<SHAPE>* wo = wouts<SHAPE>();
     const int NW = T >> 5;
-    for (int e = lane; e < N * N; e += 32) {
-      const int a = e / N, b = e - a * N;
-      const int i = P.slot[a], j = P.slot[b];
-      const int lo = min(i, j), hi = max(i, j);
+    // the sums of the upper triangle, one per lane, into both halves
+#pragma unroll 1
+    for (int e = lane; e < L::NP; e += 32) {
+      int lo = 0, hi = e;
+#pragma unroll 1
+      while (hi >= L::NS - lo) hi -= L::NS - lo++;
+      hi += lo;
       double m = 0.0, er = 0.0;
-      for (int w = hw0; w < hw0 + hnw; ++w) m += wo[w].M[lo * L::VW + hi];
-      for (int w = hw0; w < hw0 + hnw; ++w) er += wo[w].E[pair_index(lo, hi, L::NS)];
-      c.H[e] = m - er;
+#pragma unroll 1
+      for (int w = hw0; w < hw0 + hnw; ++w) {
+        m += wo[w].M[lo * L::VW + hi];
+        er += wo[w].E[e];
+      }
+      const int a = P.cidx[lo], b = P.cidx[hi];
+      if (a >= 0 && b >= 0) c.H[a * N + b] = c.H[b * N + a] = m - er;
     }
     if (lane < N) {
       double qq = 0.0;
@@ -400,69 +407,129 @@ struct Engine {
     // LU with partial pivoting in place in c.H (the unblocked DGETRF steps:
     // IDAMAX, the row swap, the scaling by the pivot's reciprocal, the rank-1
     // update), then the inverse a column per lane, x = U^-1 L^-1 P e_lane.
-    // Rolled loops over shared memory: the solve runs once per iteration on
-    // one warp, and a short loop stays in the instruction cache.
+    // Loops over shared memory: the solve runs once per iteration on one
+    // warp, and a short loop stays in the instruction cache.
     int info = 0;
-#pragma unroll 1
-    for (int j = 0; j < N; ++j) {
-      double best = fabs(c.H[j * N + j]);
-      int p = j;
-#pragma unroll 1
-      for (int i = j + 1; i < N; ++i) {
-        const double ai = fabs(c.H[i * N + j]);
-        if (ai > best) { best = ai; p = i; }
-      }
-      const double pv = c.H[p * N + j];
-      __syncwarp();
-      if (lane == 0) c.piv[j] = p;
-      if (pv != 0.0) {
-        if (p != j && lane < N) {
-          const double t = c.H[j * N + lane];
-          c.H[j * N + lane] = c.H[p * N + lane];
-          c.H[p * N + lane] = t;
-        }
-        __syncwarp();
-        const double r = 1.0 / pv;
-        if (lane > j && lane < N) c.H[lane * N + j] = c.H[lane * N + j] * r;
-      } else if (info == 0) {
-        info = j + 1;
-      }
-      __syncwarp();
-      const int m = N - 1 - j;
-#pragma unroll 1
-      for (int e = lane; e < m * m; e += 32) {
-        const int i = j + 1 + e / m, kx = j + 1 + (e - (e / m) * m);
-        c.H[i * N + kx] = c.H[i * N + kx] - c.H[i * N + j] * c.H[j * N + kx];
-      }
-      __syncwarp();
-    }
-    if (info == 0 && lane < N) {
-      double* x = ctl_inv<SHAPE>(c) + lane;     // column `lane`, stride N
-      int pos = lane;                           // P e_lane is a unit vector
+    if constexpr (SHAPE != DICEGPU_QUADRATIC_SF) {
+      // lane l updates entry (1 + l / 5, 1 + l mod 5); the pivot is found by
+      // reductions over the lanes (the first largest magnitude; a NaN is taken
+      // only where it stands first, as IDAMAX's comparisons leave it)
+      const int ri = 1 + lane / 5, ck = 1 + lane % 5;
+      int pos = lane;   // the row of P e_lane's unit entry
 #pragma unroll 1
       for (int j = 0; j < N; ++j) {
-        const int pj = c.piv[j];
-        if (pos == j) pos = pj;
-        else if (pos == pj) pos = j;
+        unsigned long long key = 0ull;
+        if (lane >= j && lane < N) {
+          key = (unsigned long long)__double_as_longlong(c.H[lane * N + j]) & 0x7fffffffffffffffull;
+          if (key > 0x7ff0000000000000ull && lane != j) key = 0ull;
+        }
+        const unsigned kh = (unsigned)(key >> 32), mh = __reduce_max_sync(FULL, kh);
+        const unsigned kl = kh == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(FULL, kl);
+        const int p = __ffs(__ballot_sync(FULL, lane >= j && lane < N && kh == mh && kl == ml)) - 1;
+        const double pv = c.H[p * N + j];
+        if (pos == j) pos = p;
+        else if (pos == p) pos = j;
+        if (pv != 0.0) {
+          const double rp = 1.0 / pv;
+          if (p != j && lane < N) {
+            const double t = c.H[j * N + lane];
+            c.H[j * N + lane] = c.H[p * N + lane];
+            c.H[p * N + lane] = t;
+          }
+          __syncwarp();
+          if (lane > j && lane < N) c.H[lane * N + j] = c.H[lane * N + j] * rp;
+        } else if (info == 0) {
+          info = j + 1;
+        }
+        __syncwarp();
+        if (ri > j && ck > j && ri < N && ck < N)
+          c.H[ri * N + ck] = c.H[ri * N + ck] - c.H[ri * N + j] * c.H[j * N + ck];
+        __syncwarp();
       }
-#pragma unroll 1
-      for (int i = 0; i < N; ++i) x[i * N] = i == pos ? 1.0 : 0.0;
-#pragma unroll 1
-      for (int i = 1; i < N; ++i) {
-        double acc = x[i * N];
-#pragma unroll 1
-        for (int j = 0; j < i; ++j) acc = acc - c.H[i * N + j] * x[j * N];
-        x[i * N] = acc;
+      if (info == 0 && lane < N) {
+        double x[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          double acc = i == pos ? 1.0 : 0.0;
+#pragma unroll
+          for (int j = 0; j < i; ++j)
+            if (i < N) acc = acc - c.H[i * N + j] * x[j];
+          x[i] = acc;
+        }
+#pragma unroll
+        for (int i = 5; i >= 0; --i) {
+          if (i >= N) continue;
+          double acc = x[i];
+#pragma unroll
+          for (int j = i + 1; j < 6; ++j)
+            if (j < N) acc = acc - c.H[i * N + j] * x[j];
+          x[i] = acc / c.H[i * N + i];
+          ctl_inv<SHAPE>(c)[i * N + lane] = x[i];
+        }
       }
+      __syncwarp();
+    } else {
 #pragma unroll 1
-      for (int i = N - 1; i >= 0; --i) {
-        double acc = x[i * N];
+      for (int j = 0; j < N; ++j) {
+        double best = fabs(c.H[j * N + j]);
+        int p = j;
 #pragma unroll 1
-        for (int j = i + 1; j < N; ++j) acc = acc - c.H[i * N + j] * x[j * N];
-        x[i * N] = acc / c.H[i * N + i];
+        for (int i = j + 1; i < N; ++i) {
+          const double ai = fabs(c.H[i * N + j]);
+          if (ai > best) { best = ai; p = i; }
+        }
+        const double pv = c.H[p * N + j];
+        __syncwarp();
+        if (lane == 0) c.piv[j] = p;
+        if (pv != 0.0) {
+          if (p != j && lane < N) {
+            const double t = c.H[j * N + lane];
+            c.H[j * N + lane] = c.H[p * N + lane];
+            c.H[p * N + lane] = t;
+          }
+          __syncwarp();
+          const double r = 1.0 / pv;
+          if (lane > j && lane < N) c.H[lane * N + j] = c.H[lane * N + j] * r;
+        } else if (info == 0) {
+          info = j + 1;
+        }
+        __syncwarp();
+        const int m = N - 1 - j;
+#pragma unroll 1
+        for (int e = lane; e < m * m; e += 32) {
+          const int i = j + 1 + e / m, kx = j + 1 + (e - (e / m) * m);
+          c.H[i * N + kx] = c.H[i * N + kx] - c.H[i * N + j] * c.H[j * N + kx];
+        }
+        __syncwarp();
       }
+      if (info == 0 && lane < N) {
+        double* x = ctl_inv<SHAPE>(c) + lane;     // column `lane`, stride N
+        int pos = lane;                           // P e_lane is a unit vector
+#pragma unroll 1
+        for (int j = 0; j < N; ++j) {
+          const int pj = c.piv[j];
+          if (pos == j) pos = pj;
+          else if (pos == pj) pos = j;
+        }
+#pragma unroll 1
+        for (int i = 0; i < N; ++i) x[i * N] = i == pos ? 1.0 : 0.0;
+#pragma unroll 1
+        for (int i = 1; i < N; ++i) {
+          double acc = x[i * N];
+#pragma unroll 1
+          for (int j = 0; j < i; ++j) acc = acc - c.H[i * N + j] * x[j * N];
+          x[i * N] = acc;
+        }
+#pragma unroll 1
+        for (int i = N - 1; i >= 0; --i) {
+          double acc = x[i * N];
+#pragma unroll 1
+          for (int j = i + 1; j < N; ++j) acc = acc - c.H[i * N + j] * x[j * N];
+          x[i * N] = acc / c.H[i * N + i];
+        }
+      }
+      __syncwarp();
     }
-    __syncwarp();
     bool notc = false;
     float nw = 0.0f;
     if (lane < N) {

@@ -487,7 +487,8 @@ __device__ __forceinline__ void cta_pass(const PassInT<MASKED> in, const MapCons
     if (MASKED && live) live = !mv.hides(px, py);
     float G = 0.0f, gx = 0.0f, gy = 0.0f;
     if (live) {
-      if (GRADS && DEFGRAD) interp_ref<INTERP, true>(in.def, mx, my, G, gx, gy);
+      if (GRADS && DEFGRAD && INTERP == DICEGPU_KEYS_FOURTH) keys_ref_rows(in.def, mx, my, G, gx, gy);
+      else if (GRADS && DEFGRAD) interp_ref<INTERP, true>(in.def, mx, my, G, gx, gy);
       else interp_ref<INTERP, false>(in.def, mx, my, G, gx, gy);
       if (GRADS && !DEFGRAD) {
         gx = rin ? __ldg(in.refgx + ri) : 0.0f;

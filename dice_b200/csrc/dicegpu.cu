@@ -315,6 +315,8 @@ static int build_devparams(const dicegpu_params& p, DevParams& d) {
     d.deltas[1] = (float)p.robust_delta_disp;
     d.has_rot = p.enable_rotation ? 1 : 0;
   }
+  for (int i = 0; i < 12; ++i) d.cidx[i] = -1;
+  for (int k = 0; k < d.N; ++k) d.cidx[d.slot[k]] = k;
   d.interp = p.interpolation;
   d.opt = p.optimization;
   d.max_fast = p.max_solver_iterations_fast;
