@@ -11,11 +11,15 @@
 // rounded to float as the reference stores them.
 //
 // The neighbours come from a uniform grid of cell size >= the radius (3 x 3
-// cells cover the disc) whose per-subset floats are packed in cell order
-// (vsg_pack_kernel).  A warp accumulates the twelve double sums of X^T X,
-// X^T u and X^T v for 32 subsets in turn, then each lane solves one
-// subset's 3 x 3 system by LU with partial pivoting and an explicit inverse
-// (the reference's GETRF / GETRI).
+// cells cover the disc) whose per-subset values are packed in cell order
+// (vsg_pack_kernel).  A thread takes one subset, in cell order: the three
+// cells of a grid row are one contiguous run of the packed array, the lanes of
+// a warp read nearly the same runs, and each keeps its own twelve sums of
+// X^T X, X^T u and X^T v and solves its 3 x 3 system by LU with partial
+// pivoting and an explicit inverse (the reference's GETRF / GETRI).  The sums
+// are exact for the reference's integer centres unless displacements span more
+// than about 2^9, so their order does not show.  (With a warp per subset
+// at a time, twelve warp-wide double sums each, 158,404 subsets took 265 us.)
 // The condition number is computed exactly where the reference estimates it
 // (GECON); the two differ only for nearly collinear neighbourhoods.
 #pragma once
@@ -29,7 +33,9 @@ struct VsgArgs {
   const int32_t* cell_off;   // [ncx * ncy + 1] into cell_pts / packed
   const int32_t* cell_pts;   // subset indices grouped by cell
   const int32_t* pos_of;     // position of each subset in cell order
-  float4* packed;            // per position: x (NaN when sigma < 0), y, u, v as floats
+  const float2* centre;      // per position: x, y
+  float2* packed;            // per position: x (NaN when sigma < 0), y
+  double2* packed_uv;        // per position: u, v as floats, widened
   int ncx, ncy;
   float x0, y0, cell;        // grid origin and cell size
   float r2;                  // r^2 + 1e-5
@@ -44,16 +50,19 @@ __global__ void __launch_bounds__(256) vsg_pack_kernel(VsgArgs a) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
     const double* f = a.fields + (size_t)i * DICEGPU_FIELD_STRIDE;
     const bool valid = (float)f[DICEGPU_F_SIGMA] >= 0.0f;
-    a.packed[a.pos_of[i]] = make_float4(valid ? (float)f[DICEGPU_F_COORD_X] : __int_as_float(0x7fc00000),
-                                        (float)f[DICEGPU_F_COORD_Y], (float)f[DICEGPU_F_DISP_X],
-                                        (float)f[DICEGPU_F_DISP_Y]);
+    const int p = a.pos_of[i];
+    a.packed[p] = make_float2(valid ? (float)f[DICEGPU_F_COORD_X] : __int_as_float(0x7fc00000),
+                              (float)f[DICEGPU_F_COORD_Y]);
+    a.packed_uv[p] = make_double2((double)(float)f[DICEGPU_F_DISP_X], (double)(float)f[DICEGPU_F_DISP_Y]);
   }
 }
 
-__device__ __forceinline__ double vsg_warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+// the subsets' centres, packed
+__global__ void vsg_coords_kernel(const double* __restrict__ fields, int n, double2* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n)
+    out[i] = make_double2(fields[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_X],
+                          fields[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_Y]);
 }
 
 // LU with partial pivoting and the inverse of a 3 x 3; false on a zero pivot
@@ -96,86 +105,62 @@ __device__ inline double vsg_norm1(const double M[3][3]) {
   return a;
 }
 
-// One warp per batch of 32 subsets.  For each subset of the batch the lanes
-// take its candidates in turn (the three cells of a grid row are one
-// contiguous run of the packed array) and the twelve double sums are reduced
-// across the warp; lane k keeps subset k's sums, and the 32 solves then run
-// in parallel, one per lane.
-__global__ void __launch_bounds__(256) vsg_kernel(VsgArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < a.n; base += nwarps * 32) {
-    const int cnt = min(32, a.n - base);
-    double m[12];
+__global__ void __launch_bounds__(128) vsg_kernel(VsgArgs a) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 >= a.n) return;
+  const float2 ci = a.centre[t0];
+  const float xi = ci.x, yi = ci.y;
+  const bool self = !isnan(a.packed[t0].x);
+  const int gx = (int)floorf((xi - a.x0) / a.cell), gy = (int)floorf((yi - a.y0) / a.cell);
+  // sums: dx, dy, dx dx, dx dy, dy dy, u, dx u, dy u, v, dx v, dy v
+  double s[11];
 #pragma unroll
-    for (int k = 0; k < 12; ++k) m[k] = 0.0;
-    int mvalid = 0;
-    bool mself = false;
-    for (int k = 0; k < cnt; ++k) {
-      const int i = base + k;
-      const double* fi = a.fields + (size_t)i * DICEGPU_FIELD_STRIDE;
-      const float xi = (float)fi[DICEGPU_F_COORD_X], yi = (float)fi[DICEGPU_F_COORD_Y];
-      const int gx = (int)floorf((xi - a.x0) / a.cell), gy = (int)floorf((yi - a.y0) / a.cell);
-      // sums: n, dx, dy, dx dx, dx dy, dy dy, u, dx u, dy u, v, dx v, dy v
-      double s[12];
-#pragma unroll
-      for (int q = 0; q < 12; ++q) s[q] = 0.0;
-      int valid = 0;
-      const int cx0 = max(gx - 1, 0), cx1 = min(gx + 1, a.ncx - 1);
-      for (int cy = max(gy - 1, 0); cy <= min(gy + 1, a.ncy - 1); ++cy) {
-        const int t1 = a.cell_off[cy * a.ncx + cx1 + 1];
-        for (int t = a.cell_off[cy * a.ncx + cx0] + lane; t < t1; t += 32) {
-          const float4 pj = __ldg(a.packed + t);
-          const float ex = __fsub_rn(xi, pj.x), ey = __fsub_rn(yi, pj.y);
-          const float d2 = __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey));
-          if (!(d2 < a.r2)) continue;   // also an invalid neighbour (x = NaN)
-          const double dx = (double)__fsub_rn(pj.x, xi), dy = (double)__fsub_rn(pj.y, yi);
-          const double u = (double)pj.z, v = (double)pj.w;
-          ++valid;
-          s[0] += 1.0; s[1] += dx; s[2] += dy;
-          s[3] = fma(dx, dx, s[3]); s[4] = fma(dx, dy, s[4]); s[5] = fma(dy, dy, s[5]);
-          s[6] += u; s[7] = fma(dx, u, s[7]); s[8] = fma(dy, u, s[8]);
-          s[9] += v; s[10] = fma(dx, v, s[10]); s[11] = fma(dy, v, s[11]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 12; ++q) s[q] = vsg_warp_sum(s[q]);
-      for (int o = 16; o > 0; o >>= 1) valid += __shfl_xor_sync(0xffffffffu, valid, o);
-      if (lane == k) {
-#pragma unroll
-        for (int q = 0; q < 12; ++q) m[q] = s[q];
-        mvalid = valid;
-        mself = (float)fi[DICEGPU_F_SIGMA] >= 0.0f;
-      }
+  for (int q = 0; q < 11; ++q) s[q] = 0.0;
+  int valid = 0;
+  const int cx0 = max(gx - 1, 0), cx1 = min(gx + 1, a.ncx - 1);
+  for (int cy = max(gy - 1, 0); cy <= min(gy + 1, a.ncy - 1); ++cy) {
+    const int t1 = a.cell_off[cy * a.ncx + cx1 + 1];
+    for (int t = a.cell_off[cy * a.ncx + cx0]; t < t1; ++t) {
+      const float2 pj = __ldg(a.packed + t);
+      const float ex = __fsub_rn(xi, pj.x), ey = __fsub_rn(yi, pj.y);
+      const float d2 = __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey));
+      if (!(d2 < a.r2)) continue;   // also an invalid neighbour (x = NaN)
+      const double2 uv = __ldg(a.packed_uv + t);
+      const double dx = -(double)ex, dy = -(double)ey;   // pj - i, rounded alike
+      ++valid;
+      s[0] += dx; s[1] += dy;
+      s[2] = fma(dx, dx, s[2]); s[3] = fma(dx, dy, s[3]); s[4] = fma(dy, dy, s[4]);
+      s[5] += uv.x; s[6] = fma(dx, uv.x, s[6]); s[7] = fma(dy, uv.x, s[7]);
+      s[8] += uv.y; s[9] = fma(dx, uv.y, s[9]); s[10] = fma(dy, uv.y, s[10]);
     }
-    if (lane >= cnt) continue;
-    const int i = base + lane;
-    double* o = a.out + (size_t)i * DICEGPU_VSG_STRIDE;
-    double r[7] = {0, 0, 0, 0, 0, 0, 0};
-    bool ok = mself && mvalid >= 3;
-    if (ok) {
-      const double XtX[3][3] = {{m[0], m[1], m[2]}, {m[1], m[3], m[4]}, {m[2], m[4], m[5]}};
-      double inv[3][3];
-      ok = vsg_inverse3(XtX, inv);
-      if (ok) ok = !(1.0 / (vsg_norm1(XtX) * vsg_norm1(inv)) < 1.0e-12);
-      if (ok) {
-        const double Xu[3] = {m[6], m[7], m[8]}, Xv[3] = {m[9], m[10], m[11]};
-        double cu[3], cv[3];
-        for (int p = 0; p < 3; ++p) {
-          cu[p] = inv[p][0] * Xu[0] + inv[p][1] * Xu[1] + inv[p][2] * Xu[2];
-          cv[p] = inv[p][0] * Xv[0] + inv[p][1] * Xv[1] + inv[p][2] * Xv[2];
-        }
-        const double dudx = cu[1], dudy = cu[2], dvdx = cv[1], dvdy = cv[2];
-        r[0] = (float)(0.5 * (2.0 * dudx + dudx * dudx + dvdx * dvdx));
-        r[1] = (float)(0.5 * (2.0 * dvdy + dudy * dudy + dvdy * dvdy));
-        r[2] = (float)(0.5 * (dudy + dvdx + dudx * dudy + dvdx * dvdy));
-        r[3] = (float)dudx; r[4] = (float)dudy; r[5] = (float)dvdx; r[6] = (float)dvdy;
-      }
-    }
-    for (int k = 0; k < 7; ++k) o[k] = r[k];
-    o[DICEGPU_VSG_NEIGHBORS] = mvalid;
-    if (!ok) a.fields[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_MATCH] = -1.0;
   }
+  const int i = a.cell_pts[t0];
+  double* o = a.out + (size_t)i * DICEGPU_VSG_STRIDE;
+  double r[7] = {0, 0, 0, 0, 0, 0, 0};
+  bool ok = self && valid >= 3;
+  if (ok) {
+    const double XtX[3][3] = {{(double)valid, s[0], s[1]}, {s[0], s[2], s[3]}, {s[1], s[3], s[4]}};
+    double inv[3][3];
+    ok = vsg_inverse3(XtX, inv);
+    if (ok) ok = !(1.0 / (vsg_norm1(XtX) * vsg_norm1(inv)) < 1.0e-12);
+    if (ok) {
+      const double Xu[3] = {s[5], s[6], s[7]}, Xv[3] = {s[8], s[9], s[10]};
+      double cu[3], cv[3];
+      for (int p = 0; p < 3; ++p) {
+        cu[p] = inv[p][0] * Xu[0] + inv[p][1] * Xu[1] + inv[p][2] * Xu[2];
+        cv[p] = inv[p][0] * Xv[0] + inv[p][1] * Xv[1] + inv[p][2] * Xv[2];
+      }
+      const double dudx = cu[1], dudy = cu[2], dvdx = cv[1], dvdy = cv[2];
+      r[0] = (float)(0.5 * (2.0 * dudx + dudx * dudx + dvdx * dvdx));
+      r[1] = (float)(0.5 * (2.0 * dvdy + dudy * dudy + dvdy * dvdy));
+      r[2] = (float)(0.5 * (dudy + dvdx + dudx * dudy + dvdx * dvdy));
+      r[3] = (float)dudx; r[4] = (float)dudy; r[5] = (float)dvdx; r[6] = (float)dvdy;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 6; k += 2) reinterpret_cast<double2*>(o)[k / 2] = make_double2(r[k], r[k + 1]);
+  reinterpret_cast<double2*>(o)[3] = make_double2(r[6], (double)valid);
+  if (!ok) a.fields[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_MATCH] = -1.0;
 }
 
 // k nearest neighbourhoods (a negative window: Post_Processor::

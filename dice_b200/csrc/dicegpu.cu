@@ -253,7 +253,8 @@ struct dicegpu_ctx {
   int vsg_ncx = 0, vsg_ncy = 0;
   float vsg_x0 = 0.0f, vsg_y0 = 0.0f, vsg_cell = 1.0f, vsg_r2 = 0.0f;
   DevBuf<int32_t> d_vsg_cell_off, d_vsg_cell_pts, d_vsg_pos;
-  DevBuf<float4> d_vsg_packed;
+  DevBuf<float2> d_vsg_centre, d_vsg_packed;
+  DevBuf<double2> d_vsg_uv;
   DevBuf<int32_t> d_vsg_nbr;   // k nearest neighbours per subset (negative windows)
   DevBuf<double> d_vsg;
   std::vector<double> h_vsg_coords;   // the coordinates the grid was built for
@@ -437,7 +438,7 @@ extern "C" int dicegpu_destroy(dicegpu_ctx* c) {
   c->d_dv_off.release(); c->d_dvx.release(); c->d_dvy.release();
   c->d_snapshot.release();
   c->d_vsg_cell_off.release(); c->d_vsg_cell_pts.release(); c->d_vsg.release();
-  c->d_vsg_pos.release(); c->d_vsg_packed.release(); c->d_vsg_nbr.release();
+  c->d_vsg_pos.release(); c->d_vsg_packed.release(); c->d_vsg_centre.release(); c->d_vsg_uv.release(); c->d_vsg_nbr.release();
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->graph) cudaGraphDestroy(c->graph);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
@@ -1147,16 +1148,22 @@ static int ensure_blocking_desc(dicegpu_ctx* c) {
 // neighbour even when a centre sits on a cell edge.
 static int build_vsg_grid(dicegpu_ctx* c, int window) {
   const int n = c->n;
-  std::vector<double> rows((size_t)n * DICEGPU_FIELD_STRIDE);
-  CK(cudaMemcpyAsync(rows.data(), c->d_fields, rows.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  int rc;
+  if ((rc = c->d_vsg_cell_pts.ensure(n)) || (rc = c->d_vsg_pos.ensure(n)) || (rc = c->d_vsg_packed.ensure(n)) ||
+      (rc = c->d_vsg_uv.ensure(n)) || (rc = c->d_vsg_centre.ensure(n)))
+    return rc;
+  // the centres only (16 of a field row's 256 bytes), gathered on the device
+  std::vector<double> coords(2 * (size_t)n);
+  vsg_coords_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(c->d_fields, n, c->d_vsg_uv.p);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(coords.data(), c->d_vsg_uv.p, coords.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   // radius of the reference's neighbourhood search (initialize_neighborhood)
   const float rad = (float)((float)window / 2.0);
   const float r2 = rad * rad + 1.0e-5f;
   float x0 = 0.0f, y0 = 0.0f, x1 = 0.0f, y1 = 0.0f;
   for (int i = 0; i < n; ++i) {
-    const float x = (float)rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_X];
-    const float y = (float)rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_Y];
+    const float x = (float)coords[2 * (size_t)i], y = (float)coords[2 * (size_t)i + 1];
     if (!std::isfinite(x) || !std::isfinite(y)) return DICEGPU_ERR_ARG;
     if (i == 0 || x < x0) x0 = x;
     if (i == 0 || y < y0) y0 = y;
@@ -1169,8 +1176,7 @@ static int build_vsg_grid(dicegpu_ctx* c, int window) {
   const int ncx = (int)std::floor((x1 - x0) / cell) + 1, ncy = (int)std::floor((y1 - y0) / cell) + 1;
   std::vector<int32_t> off((size_t)ncx * ncy + 1, 0), pts(n), cell_of(n);
   for (int i = 0; i < n; ++i) {
-    const float x = (float)rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_X];
-    const float y = (float)rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_Y];
+    const float x = (float)coords[2 * (size_t)i], y = (float)coords[2 * (size_t)i + 1];
     const int gx = std::min(std::max((int)std::floor((x - x0) / cell), 0), ncx - 1);
     const int gy = std::min(std::max((int)std::floor((y - y0) / cell), 0), ncy - 1);
     cell_of[i] = gy * ncx + gx;
@@ -1178,25 +1184,22 @@ static int build_vsg_grid(dicegpu_ctx* c, int window) {
   }
   for (size_t k = 0; k + 1 < off.size(); ++k) off[k + 1] += off[k];
   std::vector<int32_t> pos(n);
+  std::vector<float2> centre(n);
   {
     std::vector<int32_t> fill(off.begin(), off.end() - 1);
     for (int i = 0; i < n; ++i) {
-      pos[i] = fill[cell_of[i]]++;
-      pts[pos[i]] = i;
+      const int p = fill[cell_of[i]]++;
+      pos[i] = p;
+      pts[p] = i;
+      centre[p] = make_float2((float)coords[2 * (size_t)i], (float)coords[2 * (size_t)i + 1]);
     }
   }
-  int rc;
-  if ((rc = c->d_vsg_cell_off.ensure(off.size())) || (rc = c->d_vsg_cell_pts.ensure(n)) ||
-      (rc = c->d_vsg_pos.ensure(n)) || (rc = c->d_vsg_packed.ensure(n)))
-    return rc;
+  if ((rc = c->d_vsg_cell_off.ensure(off.size()))) return rc;
   CK(cudaMemcpy(c->d_vsg_cell_off.p, off.data(), off.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_vsg_cell_pts.p, pts.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_vsg_pos.p, pos.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
-  c->h_vsg_coords.resize(2 * (size_t)n);
-  for (int i = 0; i < n; ++i) {
-    c->h_vsg_coords[2 * i] = rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_X];
-    c->h_vsg_coords[2 * i + 1] = rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_Y];
-  }
+  CK(cudaMemcpy(c->d_vsg_centre.p, centre.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
+  c->h_vsg_coords.swap(coords);
   c->vsg_ncx = ncx;
   c->vsg_ncy = ncy;
   c->vsg_x0 = x0;
@@ -1300,13 +1303,12 @@ extern "C" int dicegpu_vsg_strain(dicegpu_ctx* c, int window_size, double* out, 
   }
   if (c->vsg_window != window_size && (rc = build_vsg_grid(c, window_size))) return rc;
   if ((rc = c->d_vsg.ensure((size_t)c->n * DICEGPU_VSG_STRIDE))) return rc;
-  VsgArgs va{c->d_fields, c->n, c->d_vsg_cell_off.p, c->d_vsg_cell_pts.p, c->d_vsg_pos.p, c->d_vsg_packed.p,
-             c->vsg_ncx, c->vsg_ncy, c->vsg_x0, c->vsg_y0, c->vsg_cell, c->vsg_r2, c->d_vsg.p};
+  VsgArgs va{c->d_fields, c->n, c->d_vsg_cell_off.p, c->d_vsg_cell_pts.p, c->d_vsg_pos.p, c->d_vsg_centre.p,
+             c->d_vsg_packed.p, c->d_vsg_uv.p, c->vsg_ncx, c->vsg_ncy, c->vsg_x0, c->vsg_y0, c->vsg_cell, c->vsg_r2, c->d_vsg.p};
   const unsigned pblocks = (unsigned)std::min<int64_t>(((int64_t)c->n + 255) / 256, (int64_t)c->num_sms * 8);
   vsg_pack_kernel<<<pblocks, 256, 0, c->stream>>>(va);
-  // one warp per 32 subsets
-  const unsigned blocks = (unsigned)std::min<int64_t>(((int64_t)c->n + 255) / 256, (int64_t)c->num_sms * 16);
-  vsg_kernel<<<blocks, 256, 0, c->stream>>>(va);
+  const unsigned blocks = (unsigned)((c->n + 127) / 128);
+  vsg_kernel<<<blocks, 128, 0, c->stream>>>(va);
   CK(cudaGetLastError());
   c->launches += 2;
   if (out)
