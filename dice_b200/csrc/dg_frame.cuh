@@ -73,6 +73,7 @@ typedef void (*FrameKernelFn)(FrameArgs);
 #define DG_DECLARE_FRAME_FN(S, I, M) FrameKernelFn DG_FRAME_FN_NAME(S, I, M)(bool defgrad);
 DG_DECLARE_FRAME_FN(0, 0, 0) DG_DECLARE_FRAME_FN(0, 1, 0) DG_DECLARE_FRAME_FN(0, 2, 0)
 DG_DECLARE_FRAME_FN(1, 0, 0) DG_DECLARE_FRAME_FN(1, 1, 0) DG_DECLARE_FRAME_FN(1, 2, 0)
+DG_DECLARE_FRAME_FN(2, 0, 0) DG_DECLARE_FRAME_FN(2, 1, 0) DG_DECLARE_FRAME_FN(2, 2, 0)
 DG_DECLARE_FRAME_FN(0, 0, 1) DG_DECLARE_FRAME_FN(0, 1, 1) DG_DECLARE_FRAME_FN(0, 2, 1)
 DG_DECLARE_FRAME_FN(1, 0, 1) DG_DECLARE_FRAME_FN(1, 1, 1) DG_DECLARE_FRAME_FN(1, 2, 1)
 
@@ -82,6 +83,7 @@ DG_DECLARE_FRAME_FN(1, 0, 1) DG_DECLARE_FRAME_FN(1, 1, 1) DG_DECLARE_FRAME_FN(1,
 #define DG_DECLARE_FRAME_PROF(S, I, M) int DG_FRAME_PROF_NAME(S, I, M)(unsigned long long* acc16);
 DG_DECLARE_FRAME_PROF(0, 0, 0) DG_DECLARE_FRAME_PROF(0, 1, 0) DG_DECLARE_FRAME_PROF(0, 2, 0)
 DG_DECLARE_FRAME_PROF(1, 0, 0) DG_DECLARE_FRAME_PROF(1, 1, 0) DG_DECLARE_FRAME_PROF(1, 2, 0)
+DG_DECLARE_FRAME_PROF(2, 0, 0) DG_DECLARE_FRAME_PROF(2, 1, 0) DG_DECLARE_FRAME_PROF(2, 2, 0)
 DG_DECLARE_FRAME_PROF(0, 0, 1) DG_DECLARE_FRAME_PROF(0, 1, 1) DG_DECLARE_FRAME_PROF(0, 2, 1)
 DG_DECLARE_FRAME_PROF(1, 0, 1) DG_DECLARE_FRAME_PROF(1, 1, 1) DG_DECLARE_FRAME_PROF(1, 2, 1)
 #endif
@@ -91,14 +93,15 @@ DG_DECLARE_FRAME_PROF(1, 0, 1) DG_DECLARE_FRAME_PROF(1, 1, 1) DG_DECLARE_FRAME_P
 // Keys-4 / deformed-gradient kernel).
 inline FrameKernelFn pick_frame_kernel(int shape, int interp, bool defgrad, bool mask) {
   typedef FrameKernelFn (*Pick)(bool);
-  static const Pick table[2][3][2] = {
+  static const Pick table[3][3][2] = {
       {{DG_FRAME_FN_NAME(0, 0, 0), DG_FRAME_FN_NAME(0, 0, 1)},
        {DG_FRAME_FN_NAME(0, 1, 0), DG_FRAME_FN_NAME(0, 1, 1)},
        {DG_FRAME_FN_NAME(0, 2, 0), DG_FRAME_FN_NAME(0, 2, 1)}},
       {{DG_FRAME_FN_NAME(1, 0, 0), DG_FRAME_FN_NAME(1, 0, 1)},
        {DG_FRAME_FN_NAME(1, 1, 0), DG_FRAME_FN_NAME(1, 1, 1)},
-       {DG_FRAME_FN_NAME(1, 2, 0), DG_FRAME_FN_NAME(1, 2, 1)}}};
-  if (shape < 0 || shape > 1 || interp < 0 || interp > 2) return nullptr;
+       {DG_FRAME_FN_NAME(1, 2, 0), DG_FRAME_FN_NAME(1, 2, 1)}},
+      {{DG_FRAME_FN_NAME(2, 0, 0), nullptr}, {DG_FRAME_FN_NAME(2, 1, 0), nullptr}, {DG_FRAME_FN_NAME(2, 2, 0), nullptr}}};
+  if (shape < 0 || shape > 2 || (shape == kAffineLean && mask) || interp < 0 || interp > 2) return nullptr;
   return table[shape][interp][mask ? 1 : 0](defgrad);
 }
 

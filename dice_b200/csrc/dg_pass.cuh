@@ -49,6 +49,10 @@ static __device__ unsigned long long g_prof[16];   // per translation unit
 #define DG_PACC(i, t0)
 #endif
 
+// An affine subset stored lean: 17 bytes per pixel instead of 33.  For subsets
+// so large that their residual rows leave an SM one or two CTAs.
+constexpr int kAffineLean = 2;
+
 template <int SHAPE>
 struct Layout {
   static constexpr int NS = SHAPE == DICEGPU_QUADRATIC_SF ? 12 : 6;   // parameter slots
@@ -119,18 +123,13 @@ __host__ __device__ inline int pix_cap(int npix_max) { return (npix_max + 31) & 
 // starts on a 16-byte boundary)
 __host__ __device__ inline int pix_stride(int cap) { return cap + 4; }
 // stored per-pixel rows besides F and G: the affine residual vector r_0..r_5,
-// or the quadratic subset's gradients (its residuals are products of them)
-// Stored rows of an affine subset (DG_AFF_ROWS): 6, its residual vector;
-// 4, the gradients and the stretched offsets Dx, Dy; 2, the gradients only
-// (the sweeps form the residuals from them).
-#ifndef DG_AFF_ROWS
-#define DG_AFF_ROWS 6
-#endif
+// or the gradients, from which the sweeps form the residuals again (quadratic
+// subsets, whose residuals are products of them, and kAffineLean)
 template <int SHAPE>
 struct PixRows {
-  static constexpr int NR = SHAPE == DICEGPU_QUADRATIC_SF ? 2 : DG_AFF_ROWS;
+  static constexpr int NR = SHAPE == DICEGPU_AFFINE_SF ? 6 : 2;
   // the sweeps read the residual vector straight from the rows
-  static constexpr bool RESID = SHAPE != DICEGPU_QUADRATIC_SF && DG_AFF_ROWS == 6;
+  static constexpr bool RESID = SHAPE == DICEGPU_AFFINE_SF;
 };
 template <int SHAPE>
 struct SmemPlan {
@@ -437,7 +436,6 @@ template <int SHAPE, int INTERP, bool DEFGRAD, int KIND, bool MASKED>
 __device__ __forceinline__ void cta_pass(const PassInT<MASKED> in, const MapConst k) {
   using L = Layout<SHAPE>;
   constexpr bool GRADS = KIND != PK_GAMMA;
-  constexpr bool AFF = SHAPE != DICEGPU_QUADRATIC_SF;
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const bool use_ref_grads = !DEFGRAD;
   const float fcx = (float)in.cx, fcy = (float)in.cy;
@@ -512,10 +510,6 @@ __device__ __forceinline__ void cta_pass(const PassInT<MASKED> in, const MapCons
     } else if (GRADS) {
       A.R(0)[p] = gx;
       A.R(1)[p] = gy;
-      if (KIND == PK_GN && AFF && PixRows<SHAPE>::NR == 4) {
-        A.R(2)[p] = Dx;
-        A.R(3)[p] = Dy;
-      }
     }
   }
   // per-warp results
@@ -544,7 +538,7 @@ __device__ __forceinline__ void cta_pass(const PassInT<MASKED> in, const MapCons
 
 // The residual vector of a stored pixel formed from its stored gradients
 // (Quadratic_Shape_Function::residuals, :580-614; the affine one, :350-396,
-// with the stretched offsets stored or formed again as the pass formed them).
+// with the stretched offsets formed again as the pass formed them).
 template <int SHAPE>
 __device__ __forceinline__ void stored_residuals(const PassIn& in, const PixArrays& A, const MapConst& k, int p, int x,
                                                  int y, bool use_ref_grads, float* r) {
@@ -553,12 +547,7 @@ __device__ __forceinline__ void stored_residuals(const PassIn& in, const PixArra
     residuals_D<SHAPE>(k, dxf, dyf, dxf, dyf, A.R(0)[p], A.R(1)[p], use_ref_grads, r);
   } else {
     float Dx, Dy;
-    if (PixRows<SHAPE>::NR >= 4) {
-      Dx = A.R(2)[p];
-      Dy = A.R(3)[p];
-    } else {
-      affine_D(k, dxf, dyf, Dx, Dy);
-    }
+    affine_D(k, dxf, dyf, Dx, Dy);
     residuals_D<SHAPE>(k, dxf, dyf, Dx, Dy, A.R(0)[p], A.R(1)[p], use_ref_grads, r);
   }
 }

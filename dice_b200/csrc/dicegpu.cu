@@ -127,6 +127,11 @@ __global__ void interp_kernel(int method, int w, int h, const float* __restrict_
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
+// affine subsets are stored lean when their rows leave an SM this many CTAs or fewer
+#ifndef DG_LEAN_BELOW
+#define DG_LEAN_BELOW 3
+#endif
+
 // upper bound on the persistent grid
 static const int kMaxGrid = 8192;
 
@@ -1434,11 +1439,14 @@ static int npix_max(const dicegpu_ctx* c) {
 // dynamic shared memory of a frame CTA of `warps` warps: the control block,
 // per-warp sums, simplex state and staging (`fixed`), and the per-pixel
 // arrays (`pix`)
-static void frame_smem_bytes(const dicegpu_ctx* c, int warps, size_t* fixed, size_t* pix) {
+static void frame_smem_bytes(const dicegpu_ctx* c, int warps, size_t* fixed, size_t* pix, bool lean = false) {
   const int cap = pix_cap(npix_max(c));
   if (c->dp.shape == DICEGPU_QUADRATIC_SF) {
     *fixed = SmemPlan<DICEGPU_QUADRATIC_SF>::pix(warps);
     *pix = SmemPlan<DICEGPU_QUADRATIC_SF>::pix_bytes(cap);
+  } else if (lean) {
+    *fixed = SmemPlan<kAffineLean>::pix(warps);
+    *pix = SmemPlan<kAffineLean>::pix_bytes(cap);
   } else {
     *fixed = SmemPlan<DICEGPU_AFFINE_SF>::pix(warps);
     *pix = SmemPlan<DICEGPU_AFFINE_SF>::pix_bytes(cap);
@@ -1702,6 +1710,33 @@ static void wide_launch(dicegpu_ctx* c, FrameKernelFn fn, long n, int* warps, in
   *smem = s;
 }
 
+// A frame of large affine subsets, whose residual rows leave an SM one or two
+// CTAs of four warps, runs on the lean kernel when that fits more of them (the
+// registers allow four).  The double sums are those of the four warps either
+// way.  Frames that go to eight-warp CTAs (wide_launch) and launch shapes the
+// caller chose keep the rows.
+static bool lean_launch(dicegpu_ctx* c, FrameKernelFn* fn, int* blocks, size_t* smem) {
+  if (c->dp.shape != DICEGPU_AFFINE_SF || c->use_masks || c->shape_set || c->n <= 6L * *blocks) return false;
+  const int per_sm = *blocks / c->num_sms;
+  if (per_sm > DG_LEAN_BELOW) return false;
+  FrameKernelFn lf = pick_frame_kernel(kAffineLean, c->dp.interp, c->params.use_def_gradients != 0, false);
+  size_t fixed, pix;
+  frame_smem_bytes(c, c->warps_per_cta, &fixed, &pix, true);
+  const size_t s = fixed + pix;
+  if (!lf || s > (size_t)c->smem_optin) return false;
+  int lean_sm = 0;
+  if (cudaFuncSetAttribute((const void*)lf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lean_sm, (const void*)lf, c->warps_per_cta * 32, s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (lean_sm <= per_sm && !c->pix_in_global) return false;
+  *fn = lf;
+  *blocks = std::min(lean_sm * c->num_sms, kMaxGrid);
+  *smem = s;
+  return true;
+}
+
 static int run_waves(dicegpu_ctx* c, int kind, FrameKernelFn fn, int blocks, size_t smem) {
   int rc;
   if ((kind & 1) && (rc = ensure_blocking_desc(c))) return rc;
@@ -1795,7 +1830,8 @@ extern "C" int dicegpu_execute_correlation(dicegpu_ctx* c) {
   FrameArgs a;
   fill_args(c, a, MODE_CORRELATE);
   int warps = c->warps_per_cta;
-  wide_launch(c, fn, c->n, &warps, &blocks, &smem);
+  if (lean_launch(c, &fn, &blocks, &smem)) a.pix_scratch = nullptr;
+  else wide_launch(c, fn, c->n, &warps, &blocks, &smem);
   if ((rc = launch_frame(c, fn, a, c->n, blocks, warps, smem))) return rc;
   return frame_end(c);
 }

@@ -1,7 +1,8 @@
 // frame_inst.cu -- the frame kernels of one (shape function, interpolation,
 // mask) combination, with and without deformed-image gradients.  The
-// Makefile compiles this unit once per combination (DG_INST_SHAPE,
-// DG_INST_INTERP, DG_INST_MASK), so the twelve units build in parallel.
+// Makefile compiles this unit once per combination (DG_INST_SHAPE: affine,
+// quadratic, or affine stored lean; DG_INST_INTERP, DG_INST_MASK), so the
+// fifteen units build in parallel.
 #include "dg_frame.cuh"
 
 #if !defined(DG_INST_SHAPE) || !defined(DG_INST_INTERP) || !defined(DG_INST_MASK)
