@@ -2218,16 +2218,17 @@ extern "C" int dicegpu_adjoint(dicegpu_ctx* c, const double* d_fields, const dou
   a.value_out = d_value;
   a.dparams_out = d_dparams;
   a.ddef = d_ddef;
-  const void* fn = c->dp.shape == DICEGPU_QUADRATIC_SF ? (const void*)adjoint_kernel<DICEGPU_QUADRATIC_SF>
-                                                      : (const void*)adjoint_kernel<DICEGPU_AFFINE_SF>;
+  // square subsets a column per lane; pixel lists a pixel per lane
+  const bool quad = c->dp.shape == DICEGPU_QUADRATIC_SF;
+  void (*fn)(AdjointArgs);
+  if (c->use_lists) fn = quad ? adjoint_kernel<DICEGPU_QUADRATIC_SF> : adjoint_kernel<DICEGPU_AFFINE_SF>;
+  else fn = quad ? adjoint_square_kernel<DICEGPU_QUADRATIC_SF> : adjoint_square_kernel<DICEGPU_AFFINE_SF>;
+  const int threads = c->use_lists ? 256 : 128;
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-  const int need = (c->n + 7) / 8;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, threads, 0));
+  const int need = (c->n + threads / 32 - 1) / (threads / 32);
   const int blocks = std::max(1, std::min(std::max(per_sm, 1) * c->num_sms, need));
-  if (c->dp.shape == DICEGPU_QUADRATIC_SF)
-    adjoint_kernel<DICEGPU_QUADRATIC_SF><<<blocks, 256, 0, c->stream>>>(a);
-  else
-    adjoint_kernel<DICEGPU_AFFINE_SF><<<blocks, 256, 0, c->stream>>>(a);
+  fn<<<blocks, threads, 0, c->stream>>>(a);
   CK(cudaGetLastError());
   c->launches += 1;
   return DICEGPU_OK;
