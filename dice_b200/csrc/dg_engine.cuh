@@ -155,6 +155,10 @@ struct Engine {
   __device__ __forceinline__ void pass(const SubsetRef& sb, const float* slots) {
     MapConst k;
     make_mapconst<SHAPE>(slots, !DEFGRAD, (float)sb.cx, (float)sb.cy, k);
+    pass_at<KIND>(sb, k);
+  }
+  template <int KIND>
+  __device__ __forceinline__ void pass_at(const SubsetRef& sb, const MapConst& k) {
     const PassInMasked in = make_in(sb);
     if (MASK && sb.masked) {
       cta_pass<SHAPE, INTERP, DEFGRAD, KIND, true>(in, k);
@@ -213,8 +217,12 @@ struct Engine {
   // optionally divided by the number of active pixels (in double).
   __device__ float eval_gamma(const SubsetRef& sb, const float* slots, bool normalize,
                                          float* def_sum2 = nullptr) {
+    DG_PT(t_gpass);
     pass<PK_GAMMA>(sb, slots);
+    DG_PACC(8, t_gpass);
+    DG_PT(t_gsum);
     float g = gamma_exact(sb, def_sum2);
+    DG_PACC(9, t_gsum);
     if (normalize && sb.nact > 0) g = (float)((double)g / (double)sb.nact);
     return g;
   }
@@ -359,25 +367,35 @@ struct Engine {
     Ctl& c = ctl();
     const WarpOut<SHAPE>* wo = wouts<SHAPE>();
     const int NW = T >> 5;
-    // the sums of the upper triangle, one per lane, into both halves
+    DG_PT(t_s0);
+    // the sums of the upper triangle, one per lane, into both halves (up to
+    // seven warps hold Hessian sums, eight right-hand sides)
 #pragma unroll 1
     for (int e = lane; e < L::NP; e += 32) {
-      int lo = 0, hi = e;
+      int lo = 0, base = 0;   // row of the triangle, and its first entry
+      if constexpr (SHAPE != DICEGPU_QUADRATIC_SF) {
+        lo = (e >= 6) + (e >= 11) + (e >= 15) + (e >= 18) + (e >= 20);
+        base = lo * 6 - lo * (lo - 1) / 2;
+      } else {
 #pragma unroll 1
-      while (hi >= L::NS - lo) hi -= L::NS - lo++;
-      hi += lo;
-      double m = 0.0, er = 0.0;
-#pragma unroll 1
-      for (int w = hw0; w < hw0 + hnw; ++w) {
-        m += wo[w].M[lo * L::VW + hi];
-        er += wo[w].E[e];
+        while (e >= base + L::NS - lo) base += L::NS - lo++;
       }
+      const int hi = e - base + lo;
+      double m = 0.0, er = 0.0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+        if (w < hnw) {
+          m += wo[hw0 + w].M[lo * L::VW + hi];
+          er += wo[hw0 + w].E[e];
+        }
       const int a = P.cidx[lo], b = P.cidx[hi];
       if (a >= 0 && b >= 0) c.H[a * N + b] = c.H[b * N + a] = m - er;
     }
     if (lane < N) {
       double qq = 0.0;
-      for (int w = 0; w < NW; ++w) qq += wo[w].q[P.slot[lane]];
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+        if (w < NW) qq += wo[w].q[P.slot[lane]];
       c.q[lane] = qq;
     }
     __syncwarp();
@@ -386,6 +404,8 @@ struct Engine {
       c.H[N + 1] += (double)P.lm_alpha;
     }
     __syncwarp();
+    DG_PACC(10, t_s0);
+    DG_PT(t_s1);
     // 2x2 condition number of the displacement block
     float cond = -1.0f;
     {
@@ -404,6 +424,8 @@ struct Engine {
       if (lane == 0) c.status = DICEGPU_HESSIAN_SINGULAR;
       return;
     }
+    DG_PACC(11, t_s1);
+    DG_PT(t_s2);
     // LU with partial pivoting in place in c.H (the unblocked DGETRF steps:
     // IDAMAX, the row swap, the scaling by the pivot's reciprocal, the rank-1
     // update), then the inverse a column per lane, x = U^-1 L^-1 P e_lane.
@@ -446,28 +468,46 @@ struct Engine {
           c.H[ri * N + ck] = c.H[ri * N + ck] - c.H[ri * N + j] * c.H[j * N + ck];
         __syncwarp();
       }
+      DG_PACC(12, t_s2);
+      DG_PT(t_s3);
       if (info == 0 && lane < N) {
-        double x[6];
+        double* inv = ctl_inv<SHAPE>(c) + lane;   // column `lane`, stride N
+        if (N == 6) {
+          double x[6];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) {
-          double acc = i == pos ? 1.0 : 0.0;
+          for (int i = 0; i < 6; ++i) {
+            double acc = i == pos ? 1.0 : 0.0;
 #pragma unroll
-          for (int j = 0; j < i; ++j)
-            if (i < N) acc = acc - c.H[i * N + j] * x[j];
-          x[i] = acc;
-        }
+            for (int j = 0; j < i; ++j) acc = acc - c.H[i * 6 + j] * x[j];
+            x[i] = acc;
+          }
 #pragma unroll
-        for (int i = 5; i >= 0; --i) {
-          if (i >= N) continue;
-          double acc = x[i];
+          for (int i = 5; i >= 0; --i) {
+            double acc = x[i];
 #pragma unroll
-          for (int j = i + 1; j < 6; ++j)
-            if (j < N) acc = acc - c.H[i * N + j] * x[j];
-          x[i] = acc / c.H[i * N + i];
-          ctl_inv<SHAPE>(c)[i * N + lane] = x[i];
+            for (int j = i + 1; j < 6; ++j) acc = acc - c.H[i * 6 + j] * x[j];
+            x[i] = acc / c.H[i * 6 + i];
+            inv[i * 6] = x[i];
+          }
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < N; ++i) {
+            double acc = i == pos ? 1.0 : 0.0;
+#pragma unroll 1
+            for (int j = 0; j < i; ++j) acc = acc - c.H[i * N + j] * inv[j * N];
+            inv[i * N] = acc;
+          }
+#pragma unroll 1
+          for (int i = N - 1; i >= 0; --i) {
+            double acc = inv[i * N];
+#pragma unroll 1
+            for (int j = i + 1; j < N; ++j) acc = acc - c.H[i * N + j] * inv[j * N];
+            inv[i * N] = acc / c.H[i * N + i];
+          }
         }
       }
       __syncwarp();
+      DG_PACC(13, t_s3);
     } else {
 #pragma unroll 1
       for (int j = 0; j < N; ++j) {
@@ -530,12 +570,15 @@ struct Engine {
       }
       __syncwarp();
     }
+    DG_PT(t_s4);
     bool notc = false;
     float nw = 0.0f;
     if (lane < N) {
       const double* Mrow = info == 0 ? ctl_inv<SHAPE>(c) + lane * N : &c.H[lane * N];
       float du = 0.0f;
-      for (int j = 0; j < N; ++j) du = (float)((double)du + (Mrow[j] * (-1.0)) * c.q[j]);
+#pragma unroll
+      for (int j = 0; j < L::NS; ++j)
+        if (j < N) du = (float)((double)du + (Mrow[j] * (-1.0)) * c.q[j]);
       if (P.momentum != 0.0f) {
         du = du + P.momentum * c.upd_old[lane];
         c.upd_old[lane] = du;
@@ -560,6 +603,7 @@ struct Engine {
       c.status = DICEGPU_CORRELATION_SUCCESSFUL;
       c.conv = conv ? 1 : 0;
     }
+    DG_PACC(14, t_s4);
   }
 
   // --------------------------------------------------------------------------
@@ -585,11 +629,11 @@ struct Engine {
     for (; solve_it <= P.max_fast; ++solve_it) {
       num_iterations = solve_it;
       DG_PT(t_pass);
-      pass<PK_GN>(sb, slots);
-      DG_PACC(1, t_pass);
-      const int n = c.n;
       MapConst k;
       make_mapconst<SHAPE>(slots, !DEFGRAD, (float)sb.cx, (float)sb.cy, k);
+      pass_at<PK_GN>(sb, k);
+      DG_PACC(1, t_pass);
+      const int n = c.n;
       const PassInMasked in = make_in(sb);
       const PassIn& inb = static_cast<const PassIn&>(in);
       const bool fresh = solve_it == 0 && !have_state;
@@ -641,107 +685,61 @@ struct Engine {
   }
 
   // --------------------------------------------------------------------------
-  // Nelder-Mead (Simplex::minimize, DICe_Simplex.cpp:60-277).  The vertex
-  // table and sums live in the warp's SimplexState (lane 0 writes after a
-  // __syncwarp, all lanes read after the next); every warp keeps an
-  // identical copy and all evaluate the same points together.  `slots`
-  // in/out: left at the last evaluated point, as the reference's aliasing
-  // of variables and shape-function parameters leaves it
-  // (DICe_LocalShapeFunction.h:259-261); `lastp` receives that point in slot
-  // form.  The reference evaluates gamma once more at the point it evaluated
-  // last before each convergence test; that value is the last one computed,
-  // which is taken instead of a second pass.
+  // Nelder-Mead (Simplex::minimize, DICe_Simplex.cpp:60-277), every warp on
+  // its own copy, so that all take the same branches and evaluate the same
+  // points together.  Lane j holds component j of the points and sums (the
+  // vertices in the warp's SimplexState, where it reads and writes its own
+  // column), lane i the value at vertex i; what all lanes need comes by
+  // shuffles.  (With every thread keeping all components, the bookkeeping took
+  // 30 % of a simplex subset's time.)  `slots` in/out: left at the last
+  // evaluated point, as the reference's aliasing of variables and
+  // shape-function parameters leaves it (DICe_LocalShapeFunction.h:259-261).
+  // The reference evaluates gamma once more at the point it evaluated last
+  // before each convergence test; that value is the last one computed, which
+  // is taken instead of a second pass.
   // --------------------------------------------------------------------------
-  __device__ __forceinline__ void comp_to_slots(const SimplexState& S, const float* comp, float* out) const {
-    // out[s] = base[s], then the compact parameters in their slots
-#pragma unroll
-    for (int s = 0; s < 12; ++s) {
-      float v = S.base[s];
-#pragma unroll
-      for (int kx = 0; kx < 12; ++kx)
-        if (kx < A.P.N && A.P.slot[kx] == s) v = comp[kx];
-      out[s] = v;
-    }
-  }
-
   // Out of line, as beta is: these fallback paths inlined into the
   // correlation loop enlarge the code the Gauss-Newton iterations run
   // through (instruction-cache misses) and slow every subset.
-  __device__ __noinline__ int simplex(const SubsetRef& sb, float* slots, int& num_iterations, float* lastp) {
+  __device__ __noinline__ int simplex(const SubsetRef& sb, float* slots, int& num_iterations) {
     const DevParams& P = A.P;
-    const int nd = P.N;
-    const int mpts = nd + 1;
-    SimplexState& S = sx_state<SHAPE>();
-    const bool w0 = lane == 0;
-    float init[12];
+    const int nd = P.N, mpts = nd + 1;
+    float* col = sx_state<SHAPE>().pts + (lane < 12 ? lane : 0);   // vertex i's component: col[12 * i]
+    const bool comp = lane < nd;
+    float base = 0.0f;   // lane s: the slot's value at the start
 #pragma unroll
-    for (int kx = 0; kx < 12; ++kx) {
-      float v = 0.0f;
+    for (int s = 0; s < 12; ++s)
+      if (lane == s) base = slots[s];
+    const float init = __shfl_sync(FULL, base, comp ? P.slot[lane] : 0);
+    float gv = 0.0f, last_y = 0.0f, psum = 0.0f;
+    auto evaluate = [&](float v) -> float {
 #pragma unroll
-      for (int s = 0; s < 12; ++s)
-        if (kx < nd && P.slot[kx] == s) v = slots[s];
-      init[kx] = v;
-    }
-    __syncwarp();
-    if (w0) {
-#pragma unroll
-      for (int s = 0; s < 12; ++s) S.base[s] = slots[s];
-#pragma unroll
-      for (int kx = 0; kx < 12; ++kx) S.init[kx] = init[kx];
-    }
-    __syncwarp();
-    float cur[12];   // the last evaluated point (compact)
-#pragma unroll
-    for (int kx = 0; kx < 12; ++kx) cur[kx] = init[kx];
-    float last_y = 0.0f;
-    auto evaluate = [&](const float* comp) -> float {
-#pragma unroll
-      for (int kx = 0; kx < 12; ++kx) cur[kx] = comp[kx];
-      comp_to_slots(S, comp, lastp);
-      last_y = eval_gamma(sb, lastp, P.normalize_gamma != 0);
+      for (int s = 0; s < 12; ++s) {
+        const int a = P.cidx[s];
+        slots[s] = __shfl_sync(FULL, a >= 0 ? v : base, a >= 0 ? a : s);
+      }
+      last_y = eval_gamma(sb, slots, P.normalize_gamma != 0);
       return last_y;
     };
-    auto finish = [&]() { comp_to_slots(S, cur, slots); };
+    auto sum_vertices = [&]() {
+      psum = 0.0f;
+#pragma unroll 1
+      for (int i = 0; i < mpts; ++i) psum += col[12 * i];
+    };
     // initial simplex vertex_i = x0 + delta_i e_i (:82-107)
+#pragma unroll 1
     for (int i = 0; i < mpts; ++i) {
-      float v[12];
-#pragma unroll
-      for (int j = 0; j < 12; ++j) {
-        v[j] = S.init[j];
-        if (i > 0 && j == i - 1) v[j] = v[j] + P.deltas[i - 1];
-      }
-      __syncwarp();
-      if (w0) {
-#pragma unroll
-        for (int j = 0; j < 12; ++j) S.pts[i][j] = v[j];
-      }
-      __syncwarp();
+      float v = comp ? init : 0.0f;
+      if (i > 0 && lane == i - 1) v = v + P.deltas[i - 1];
+      if (lane < 12) col[12 * i] = v;
       const float g = evaluate(v);
-      __syncwarp();
-      if (w0) S.gv[i] = g;
-      __syncwarp();
+      if (lane == i) gv = g;
       if (i == 0 && g < P.skip_thr && g >= 0.0f) {
         num_iterations = 0;
-        finish();
         return DICEGPU_CORRELATION_SUCCESSFUL;
       }
     }
-    {
-      float ps[12];
-#pragma unroll
-      for (int j = 0; j < 12; ++j) {
-        float sum = 0.0f;
-        for (int i = 0; i < mpts; ++i) sum += S.pts[i][j];
-        ps[j] = sum;
-      }
-      __syncwarp();
-      if (w0) {
-#pragma unroll
-        for (int j = 0; j < 12; ++j) S.psum[j] = ps[j];
-      }
-      __syncwarp();
-    }
-    int inhi = 0;
+    sum_vertices();
     float old_rtol = 0.0f, gamma_new = 0.0f, gamma_old = -1.0f;
     int gamma_repeats = 0;
     const float tiny = 1.0e-10f;
@@ -751,45 +749,36 @@ struct Engine {
     auto trial = [&](float fac) -> float {
       const float fac1 = (float)((1.0 - (double)fac) / nd);
       const float fac2 = fac1 - fac;
-      float pt[12];
-#pragma unroll
-      for (int j = 0; j < 12; ++j) pt[j] = j < nd ? S.psum[j] * fac1 - S.pts[ihi][j] * fac2 : 0.0f;
+      const float worst = col[12 * ihi];
+      const float pt = comp ? psum * fac1 - worst * fac2 : 0.0f;
       const float y = evaluate(pt);
-      if (y < S.gv[ihi]) {
-        float ps[12];
-#pragma unroll
-        for (int j = 0; j < 12; ++j) ps[j] = S.psum[j] + (pt[j] - S.pts[ihi][j]);
-        __syncwarp();
-        if (w0) {
-          S.gv[ihi] = y;
-#pragma unroll
-          for (int j = 0; j < 12; ++j) {
-            if (j < nd) {
-              S.psum[j] = ps[j];
-              S.pts[ihi][j] = pt[j];
-            }
-          }
+      if (y < __shfl_sync(FULL, gv, ihi)) {
+        if (lane == ihi) gv = y;
+        if (comp) {
+          psum = psum + (pt - worst);
+          col[12 * ihi] = pt;
         }
-        __syncwarp();
       }
       return y;
     };
     int iteration = 0;
+#pragma unroll 1
     for (iteration = 0; iteration < P.max_robust; iteration++) {
       if (iteration >= P.max_robust - 1) {
         num_iterations = iteration;
-        finish();
         return DICEGPU_MAX_ITERATIONS_REACHED;
       }
-      int ilo = 0;
-      if (S.gv[0] > S.gv[1]) { inhi = 1; ihi = 0; } else { inhi = 0; ihi = 1; }
+      const float g0 = __shfl_sync(FULL, gv, 0), g1 = __shfl_sync(FULL, gv, 1);
+      int ilo = 0, inhi;
+      float glo = g0, ghi, gnhi;
+      if (g0 > g1) { inhi = 1; ihi = 0; gnhi = g1; ghi = g0; } else { inhi = 0; ihi = 1; gnhi = g0; ghi = g1; }
+#pragma unroll 1
       for (int i = 0; i < mpts; i++) {
-        const float gi = S.gv[i];
-        if (gi <= S.gv[ilo]) ilo = i;
-        if (gi > S.gv[ihi]) { inhi = ihi; ihi = i; }
-        else if (gi > S.gv[inhi] && i != ihi) inhi = i;
+        const float gi = __shfl_sync(FULL, gv, i);
+        if (gi <= glo) { ilo = i; glo = gi; }
+        if (gi > ghi) { inhi = ihi; gnhi = ghi; ihi = i; ghi = gi; }
+        else if (gi > gnhi && i != ihi) { inhi = i; gnhi = gi; }
       }
-      const float ghi = S.gv[ihi], glo = S.gv[ilo];
       const float rtol = (float)(2.0 * (double)fabsf(ghi - glo) / (double)(fabsf(ghi) + fabsf(glo) + tiny));
       const float rtol_diff = fabsf(rtol - old_rtol);
       old_rtol = rtol;
@@ -797,53 +786,27 @@ struct Engine {
       gamma_old = gamma_new;
       if ((double)rtol < P.robust_tol || (double)rtol_diff < P.robust_tol || gamma_repeats > 15) break;
       float ytry = trial(-1.0f);
-      if (ytry <= S.gv[ilo]) {
+      if (ytry <= __shfl_sync(FULL, gv, ilo)) {
         ytry = trial(2.0f);
-      } else if (ytry >= S.gv[inhi]) {
-        const float ysave = S.gv[ihi];
+      } else if (ytry >= __shfl_sync(FULL, gv, inhi)) {
+        const float ysave = __shfl_sync(FULL, gv, ihi);
         ytry = trial(0.5f);
         if (ytry >= ysave) {
+#pragma unroll 1
           for (int i = 0; i < mpts; i++) {
             if (i != ilo) {
-              float v[12];
-#pragma unroll
-              for (int j = 0; j < 12; ++j) v[j] = j < nd ? (float)(0.5 * (double)(S.pts[i][j] + S.pts[ilo][j])) : 0.0f;
-              __syncwarp();
-              if (w0) {
-#pragma unroll
-                for (int j = 0; j < 12; ++j) {
-                  if (j < nd) {
-                    S.pts[i][j] = v[j];
-                    S.psum[j] = v[j];
-                  }
-                }
-              }
-              __syncwarp();
+              const float v = comp ? (float)(0.5 * (double)(col[12 * i] + col[12 * ilo])) : 0.0f;
+              if (comp) col[12 * i] = v;
               const float g = evaluate(v);
-              __syncwarp();
-              if (w0) S.gv[i] = g;
-              __syncwarp();
+              if (lane == i) gv = g;
             }
           }
-          float ps[12];
-#pragma unroll
-          for (int j = 0; j < 12; ++j) {
-            float sum = 0.0f;
-            for (int i = 0; i < mpts; i++) sum += S.pts[i][j];
-            ps[j] = sum;
-          }
-          __syncwarp();
-          if (w0) {
-#pragma unroll
-            for (int j = 0; j < 12; ++j) S.psum[j] = ps[j];
-          }
-          __syncwarp();
+          sum_vertices();
         }
       }
       gamma_new = last_y;
     }
     num_iterations = iteration;
-    finish();
     return DICEGPU_CORRELATION_SUCCESSFUL;
   }
 
@@ -1080,8 +1043,7 @@ struct Engine {
       status = gauss_newton(sb, slots, false, num_iterations, cond);
       if (tid == 0) f[DICEGPU_F_CONDITION] = cond;
     } else {
-      float last_eval[12];
-      status = simplex(sb, slots, num_iterations, last_eval);
+      status = simplex(sb, slots, num_iterations);
     }
     save_shape_fields(f, slots, fcx, fcy);
     if (tid == 0) {
@@ -1361,7 +1323,6 @@ struct Engine {
     // the deformed state of the subset: none yet (Gauss-Newton then takes the
     // reference mean over all its pixels)
     bool have_state = false;
-    float last_eval[12];
     if (P.init_gamma_thr != -1.0) {
       const float g0 = eval_gamma(sb, slots, P.normalize_gamma != 0);
       have_state = true;
@@ -1384,9 +1345,9 @@ struct Engine {
       cond_set = true;
     };
     auto run_simplex = [&]() {
-      corr_status = simplex(sb, slots, num_iterations, last_eval);
+      corr_status = simplex(sb, slots, num_iterations);
       // state of the last evaluation: active set, gradients and bounding box
-      pass<PK_STATE>(sb, last_eval);
+      pass<PK_STATE>(sb, slots);
       have_state = true;
     };
     DG_PT(t_first);

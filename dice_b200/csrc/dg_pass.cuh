@@ -102,17 +102,10 @@ struct __align__(16) WarpOut {
   int n, minx, maxx, miny, maxy, pad[3];
 };
 
-// The Nelder-Mead state of Simplex::minimize (DICe_Simplex.cpp:60-277), one
-// copy per warp: every warp runs the same bookkeeping on its own copy (lane 0
-// writes, the warp reads after __syncwarp), so all warps take the same
-// branches and evaluate the same points together.
+// The vertices of Simplex::minimize (DICe_Simplex.cpp:60-277), one copy per
+// warp: vertex i's component j in pts[12 * i + j], lane j's own.
 struct __align__(16) SimplexState {
-  float pts[13][12];
-  float gv[13];
-  float psum[12];
-  float ptry[12];
-  float init[12];
-  float base[12];
+  float pts[13 * 12];
 };
 
 __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~(size_t)15; }
