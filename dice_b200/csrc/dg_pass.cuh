@@ -230,19 +230,25 @@ static __device__ __noinline__ float chain_sum(const float* a, int n, float s = 
   const float4* a4 = reinterpret_cast<const float4*>(a);
   const int nq = n >> 2;
   int q = 0;
-  if (nq >= 4) {
+  if (nq >= 12) {
+    // two sets of 16 values in turn: one is added while the other is loaded
     float4 v0 = a4[0], v1 = a4[1], v2 = a4[2], v3 = a4[3];
-    for (q = 4; q + 4 <= nq; q += 4) {
-      const float4 w0 = a4[q], w1 = a4[q + 1], w2 = a4[q + 2], w3 = a4[q + 3];
+#pragma unroll 1
+    for (; q + 12 <= nq; q += 8) {
+      const float4 w0 = a4[q + 4], w1 = a4[q + 5], w2 = a4[q + 6], w3 = a4[q + 7];
       DG_ADD4(s, v0); DG_ADD4(s, v1); DG_ADD4(s, v2); DG_ADD4(s, v3);
-      v0 = w0; v1 = w1; v2 = w2; v3 = w3;
+      v0 = a4[q + 8]; v1 = a4[q + 9]; v2 = a4[q + 10]; v3 = a4[q + 11];
+      DG_ADD4(s, w0); DG_ADD4(s, w1); DG_ADD4(s, w2); DG_ADD4(s, w3);
     }
     DG_ADD4(s, v0); DG_ADD4(s, v1); DG_ADD4(s, v2); DG_ADD4(s, v3);
+    q += 4;
   }
+#pragma unroll 1
   for (; q < nq; ++q) {
     const float4 v = a4[q];
     DG_ADD4(s, v);
   }
+#pragma unroll 1
   for (int i = nq << 2; i < n; ++i) s = __fadd_rn(s, a[i]);
   return s;
 }
@@ -274,6 +280,7 @@ static __device__ __noinline__ float chain_sum_masked(const float* a, const uint
     const float4 v = masked4(a4[q], m4[q], bit);
     DG_ADD4(s, v);
   }
+#pragma unroll 1
   for (int i = nq << 2; i < n; ++i) s = __fadd_rn(s, (m[i] & bit) ? a[i] : 0.0f);
   return s;
 }
