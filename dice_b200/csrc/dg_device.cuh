@@ -276,7 +276,7 @@ __device__ __forceinline__ void keys_ref_interior(const DevImage& im, float x, f
   gyv = c;
 }
 
-// The same value and gradients in a loop over row pairs, whose code a
+// The same value and gradients in two rounds of three rows, whose code a
 // scheduler's instruction cache holds (unrolled, the 36 taps are 5 KB, and
 // warps at different places of it wait for instructions), with the sums of I
 // and Gx as a packed pair.
@@ -290,9 +290,9 @@ __device__ __forceinline__ void keys_ref_rows(const DevImage& im, float x, float
   float c = 0.0f;
   const float4* q = im.p4 + (size_t)(iy - 2) * im.w + (ix - 2);
 #pragma unroll 1
-  for (int m = 0; m < 3; ++m) {
+  for (int m = 0; m < 2; ++m) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < 3; ++h) {
 #pragma unroll
       for (int n = 0; n < 6; ++n) {
         const float4 t = __ldg(q + n);
@@ -302,10 +302,9 @@ __device__ __forceinline__ void keys_ref_rows(const DevImage& im, float x, float
       }
       q += im.w;
     }
-    wy[0] = wy[2];
-    wy[1] = wy[3];
-    wy[2] = wy[4];
-    wy[3] = wy[5];
+    wy[0] = wy[3];
+    wy[1] = wy[4];
+    wy[2] = wy[5];
   }
   f2_unpack(ab, iv, gxv);
   gyv = c;

@@ -43,8 +43,7 @@ struct FrameArgs {
   int mode;
   int plain_index;       // >= 0: this launch processes only that subset (plain path)
   double* gamma_out;     // MODE_GAMMA output
-  int* work_counter;     // chunks handed out beyond the first gridDim.x (0 at launch)
-  int chunk;             // consecutive subsets per chunk
+  int* work_counter;     // subsets handed out beyond the first gridDim.x (0 at launch)
   int* status;           // device error word
   int32_t* passes_out;   // optional: pixel passes executed per subset (GN + simplex + epilogue)
   double* unc;           // optional: n x DICEGPU_UNCERTAINTY_STRIDE uncertainty fields

@@ -1492,7 +1492,6 @@ static void fill_args(dicegpu_ctx* c, FrameArgs& a, int mode) {
   a.mode = mode;
   a.plain_index = -1;
   a.work_counter = c->d_counter;
-  a.chunk = 1;
   a.status = c->d_status;
   a.passes_out = c->d_passes;
   a.unc = (c->params.compute_uncertainty && c->unc_n == c->n) ? c->d_unc : nullptr;
@@ -1525,12 +1524,11 @@ static int grid_for(dicegpu_ctx* c, FrameKernelFn fn, int* blocks, size_t* smem)
 }
 
 // One launch of the frame kernel over the args' subsets (`count` of them): no
-// more CTAs than there are chunks; the counter is needed beyond one chunk each.
+// more CTAs than subsets; the counter is needed beyond one subset each.
 static int launch_frame(dicegpu_ctx* c, FrameKernelFn fn, const FrameArgs& a, int count, int blocks, int warps,
                         size_t smem) {
-  const int chunks = (count + a.chunk - 1) / a.chunk;
-  blocks = std::min(blocks, chunks);
-  if (chunks > blocks) CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
+  blocks = std::min(blocks, count);
+  if (count > blocks) CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
   fn<<<blocks, warps * 32, smem, c->stream>>>(a);
   CK(cudaGetLastError());
   c->launches += 1;
