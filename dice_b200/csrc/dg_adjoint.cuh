@@ -252,7 +252,7 @@ __device__ void adjoint_subset(const AdjointArgs& A, int idx) {
   adjoint_store(A, idx, w, dp);
 }
 
-// Square subsets: a lane walks down one column of the subset (narrow subsets:
+// Square subsets with the image derivative: a lane walks down one column of the subset (narrow subsets:
 // of one of several bands of rows), a row per step, and keeps in registers the
 // 6 x 6 window of taps and the 36 sums of the scatter that the window's pixels
 // are due.  From one row to the next both slide by one row as long as no lane
@@ -379,7 +379,7 @@ __device__ void adjoint_square(const AdjointArgs& A, int idx) {
   double dp[12];
 #pragma unroll
   for (int i = 0; i < 12; ++i) dp[i] = 0.0;
-  if (w.valid && (A.dparams_out || A.ddef)) {
+  if (w.valid) {
     // pass 2: lambda_i, dObj/dp and the scatter into dObj/dI
 #pragma unroll 1
     for (int chunk = 0; chunk < c.chunks(); ++chunk) {
@@ -394,7 +394,7 @@ __device__ void adjoint_square(const AdjointArgs& A, int idx) {
       for (int r = 0; r <= c.rows; ++r) {
         c.place(r);
         const bool slide = c.slides();
-        if (A.ddef && c.had) {
+        if (c.had) {
           float* o = A.ddef + (size_t)(c.piy - 2) * c.W + (c.pix - 2);
 #pragma unroll
           for (int t = 0; t < 6; ++t) atomicAdd(o + t, acc[0][t]);
@@ -462,14 +462,12 @@ __device__ void adjoint_square(const AdjointArgs& A, int idx) {
 #pragma unroll
             for (int i = 0; i < NS; ++i) dp[i] = fma(lam, (double)rr[i], dp[i]);
           }
-          if (A.ddef) {
-            const float lf = (float)lam;
+          const float lf = (float)lam;
 #pragma unroll
-            for (int m = 0; m < 6; ++m) {
-              const float lm = lf * wy[m];
+          for (int m = 0; m < 6; ++m) {
+            const float lm = lf * wy[m];
 #pragma unroll
-              for (int t = 0; t < 6; ++t) acc[m][t] = fmaf(lm, wx[t], acc[m][t]);
-            }
+            for (int t = 0; t < 6; ++t) acc[m][t] = fmaf(lm, wx[t], acc[m][t]);
           }
         }
         c.done();

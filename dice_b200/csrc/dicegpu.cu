@@ -2216,12 +2216,21 @@ extern "C" int dicegpu_adjoint(dicegpu_ctx* c, const double* d_fields, const dou
   a.value_out = d_value;
   a.dparams_out = d_dparams;
   a.ddef = d_ddef;
-  // square subsets a column per lane; pixel lists a pixel per lane
+  // A column per lane for the image derivative of square subsets whose columns
+  // (in bands, where narrow) fill three quarters of the lanes; else a pixel
+  // per lane.  Measured, columns against pixels: 9 px (84 % of the lanes) 99 and
+  // 127 us for 17,161 subsets, 25 px (78 %) 351 and 414 for 11,664, 51 px (80 %)
+  // 390 and 552 for 3,481; but 21 px (66 %) 200 and 191 for 7,225, 41 px (64 %)
+  // 281 and 210 for 2,304; and without the image derivative, whose atomics
+  // are what the columns save, 25 px 318 and 268.
   const bool quad = c->dp.shape == DICEGPU_QUADRATIC_SF;
+  const int side = 2 * (c->params.subset_size / 2) + 1;
+  const int used = side >= 32 ? side : 32 / side * side, lanes = (used + 31) / 32 * 32;
+  const bool columns = d_ddef && !c->use_lists && 4 * used >= 3 * lanes;
   void (*fn)(AdjointArgs);
-  if (c->use_lists) fn = quad ? adjoint_kernel<DICEGPU_QUADRATIC_SF> : adjoint_kernel<DICEGPU_AFFINE_SF>;
-  else fn = quad ? adjoint_square_kernel<DICEGPU_QUADRATIC_SF> : adjoint_square_kernel<DICEGPU_AFFINE_SF>;
-  const int threads = c->use_lists ? 256 : 128;
+  if (columns) fn = quad ? adjoint_square_kernel<DICEGPU_QUADRATIC_SF> : adjoint_square_kernel<DICEGPU_AFFINE_SF>;
+  else fn = quad ? adjoint_kernel<DICEGPU_QUADRATIC_SF> : adjoint_kernel<DICEGPU_AFFINE_SF>;
+  const int threads = columns ? 128 : 256;
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, threads, 0));
   const int need = (c->n + threads / 32 - 1) / (threads / 32);

@@ -14,7 +14,7 @@ from dice_b200 import synthetic as syn
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("subset", [5, 9, 15, 25, 31, 33, 41])
+@pytest.mark.parametrize("subset", [5, 9, 15, 25, 31, 33, 41, 51, 65])
 @pytest.mark.parametrize("shape,objective,source", [(abi.AFFINE_SF, 0, 0), (abi.AFFINE_SF, 1, 1), (abi.QUADRATIC_SF, 0, 0)])
 def test_columns_equal_lists(subset, shape, objective, source):
     torch = pytest.importorskip("torch")
