@@ -539,17 +539,18 @@ int dicegpu_gauss_filter(int w, int h, const float* d_in, float* d_out, int mask
  * any device memory.  No counterpart in the reference: it exists for callers
  * that cannot call cudaMalloc -- hosts that own all device memory through
  * their own pool or budget, and per-frame loops that cannot afford the
- * device-wide wait of cudaFree.  The smoothing step's two intermediate
- * planes live in a file-scope device array of 2 * DICEGPU_NOALLOC_MAX_PIXELS
- * floats (8 MiB) that every GPU loading the library holds until exit.
+ * device-wide wait of cudaFree.  When the smoothing writes over its own
+ * input (d_gx or d_gy overlaps d_img), the input is first copied to a
+ * file-scope device array of 2 * DICEGPU_NOALLOC_MAX_PIXELS floats (8 MiB)
+ * that every GPU loading the library holds until exit.
  * With DICEGPU_CONVOLUTION_5_POINT, images larger than
  * DICEGPU_NOALLOC_MAX_PIXELS pixels are rejected with DICEGPU_ERR_ARG;
- * DICEGPU_FINITE_DIFFERENCE uses no intermediate planes and takes any size.
- * The first 5-point call on a device looks up the array's device address
+ * DICEGPU_FINITE_DIFFERENCE takes any size.
+ * The first such call on a device looks up the array's device address
  * (cudaGetSymbolAddress) and caches it per device for the process; the
  * cached address belongs to that device's context, so after a
  * cudaDeviceReset of that device it is stale and the 5-point method must not
- * be called on it again.  All calls share the one array: calls whose GPU
+ * be called on it again in place.  Such calls share the one array: those whose GPU
  * work overlaps (other streams, other host threads) race on it and must be
  * serialised by the caller.  Both image pointers are device memory. */
 #define DICEGPU_NOALLOC_MAX_PIXELS (1024 * 1024)
