@@ -29,7 +29,8 @@ namespace dg {
 // P = 8, where a row of one column per thread took 49 loads for 49.  The x
 // offsets are a rolled loop, which keeps the code within the instruction
 // cache.  P = 8 amortises the loads of large images; small ones want CTAs
-// for every SM (P = 2).
+// for every SM (P = 2).  4096^2, M = 7: 80 us, 0.55 of the rounded operations'
+// rate (one column per thread, scalar operations: 105 us).
 // ---------------------------------------------------------------------------
 struct GaussWeights {
   f32x2 c[13 * 13];   // each weight twice
@@ -139,8 +140,9 @@ __global__ void gradient_fd_kernel(int w, int h, const float* __restrict__ I, fl
 // 134 MB of planes allocated and freed for each call at 4096^2).  A thread
 // smooths eight rows of a column, both differences as one packed pair: a pair
 // read once enters up to five rows of sums with three distinct products.
-// (A warp walking down a strip without CTA barriers measured 129 us against
-// 139 at 4096^2 but 16 against 10 at 512^2.)
+// 4096^2: 95 us, 512^2: 10.5 us (tiles with flat index loops and no shared
+// products: 139 and 10.6; a warp walking down a strip without CTA barriers:
+// 129 and 16.7).
 constexpr int kSmoothB = 32, kSmoothBY = 4, kSmoothP = kSmoothB / kSmoothBY;   // 32 x 32 tile, 32 x 4 threads
 struct SmoothWeights {
   f32x2 k[3][3];   // products of 1/16, 4/16, 6/16 (exact), each twice
