@@ -20,6 +20,7 @@
 // parameter update accumulated in float.
 #pragma once
 
+#include "dg_lu.cuh"
 #include "dg_pass.cuh"
 
 namespace dg {
@@ -432,41 +433,8 @@ struct Engine {
     // warp, and a short loop stays in the instruction cache.
     int info = 0;
     if constexpr (SHAPE != DICEGPU_QUADRATIC_SF) {
-      // lane l updates entry (1 + l / 5, 1 + l mod 5); the pivot is found by
-      // reductions over the lanes (the first largest magnitude; a NaN is taken
-      // only where it stands first, as IDAMAX's comparisons leave it)
-      const int ri = 1 + lane / 5, ck = 1 + lane % 5;
-      int pos = lane;   // the row of P e_lane's unit entry
-#pragma unroll 1
-      for (int j = 0; j < N; ++j) {
-        unsigned long long key = 0ull;
-        if (lane >= j && lane < N) {
-          key = (unsigned long long)__double_as_longlong(c.H[lane * N + j]) & 0x7fffffffffffffffull;
-          if (key > 0x7ff0000000000000ull && lane != j) key = 0ull;
-        }
-        const unsigned kh = (unsigned)(key >> 32), mh = __reduce_max_sync(FULL, kh);
-        const unsigned kl = kh == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(FULL, kl);
-        const int p = __ffs(__ballot_sync(FULL, lane >= j && lane < N && kh == mh && kl == ml)) - 1;
-        const double pv = c.H[p * N + j];
-        if (pos == j) pos = p;
-        else if (pos == p) pos = j;
-        if (pv != 0.0) {
-          const double rp = 1.0 / pv;
-          if (p != j && lane < N) {
-            const double t = c.H[j * N + lane];
-            c.H[j * N + lane] = c.H[p * N + lane];
-            c.H[p * N + lane] = t;
-          }
-          __syncwarp();
-          if (lane > j && lane < N) c.H[lane * N + j] = c.H[lane * N + j] * rp;
-        } else if (info == 0) {
-          info = j + 1;
-        }
-        __syncwarp();
-        if (ri > j && ck > j && ri < N && ck < N)
-          c.H[ri * N + ck] = c.H[ri * N + ck] - c.H[ri * N + j] * c.H[j * N + ck];
-        __syncwarp();
-      }
+      int pos;   // the row of P e_lane's unit entry
+      info = lu_affine(c.H, N, lane, pos);
       DG_PACC(12, t_s2);
       DG_PT(t_s3);
       if (info == 0 && lane < N) {
