@@ -655,8 +655,8 @@ struct Engine {
   // Nelder-Mead (Simplex::minimize, DICe_Simplex.cpp:60-277), every warp on
   // its own copy, so that all take the same branches and evaluate the same
   // points together.  Lane j holds component j of the points and sums (the
-  // vertices in the warp's SimplexState, where it reads and writes its own
-  // column), lane i the value at vertex i; what all lanes need comes by
+  // vertices in the warp's SimplexState, where it alone reads and writes its
+  // column; lanes without a component touch none), lane i the value at vertex i; what all lanes need comes by
   // shuffles.  (With every thread keeping all components, the bookkeeping took
   // 30 % of a simplex subset's time.)  `slots` in/out: left at the last
   // evaluated point, as the reference's aliasing of variables and
@@ -671,8 +671,8 @@ struct Engine {
   __device__ __noinline__ int simplex(const SubsetRef& sb, float* slots, int& num_iterations) {
     const DevParams& P = A.P;
     const int nd = P.N, mpts = nd + 1;
-    float* col = sx_state<SHAPE>().pts + (lane < 12 ? lane : 0);   // vertex i's component: col[12 * i]
     const bool comp = lane < nd;
+    float* col = sx_state<SHAPE>().pts + (comp ? lane : 0);   // vertex i's component: col[12 * i]
     float base = 0.0f;   // lane s: the slot's value at the start
 #pragma unroll
     for (int s = 0; s < 12; ++s)
@@ -690,6 +690,7 @@ struct Engine {
     };
     auto sum_vertices = [&]() {
       psum = 0.0f;
+      if (!comp) return;
 #pragma unroll 1
       for (int i = 0; i < mpts; ++i) psum += col[12 * i];
     };
@@ -698,7 +699,7 @@ struct Engine {
     for (int i = 0; i < mpts; ++i) {
       float v = comp ? init : 0.0f;
       if (i > 0 && lane == i - 1) v = v + P.deltas[i - 1];
-      if (lane < 12) col[12 * i] = v;
+      if (comp) col[12 * i] = v;
       const float g = evaluate(v);
       if (lane == i) gv = g;
       if (i == 0 && g < P.skip_thr && g >= 0.0f) {
@@ -716,7 +717,7 @@ struct Engine {
     auto trial = [&](float fac) -> float {
       const float fac1 = (float)((1.0 - (double)fac) / nd);
       const float fac2 = fac1 - fac;
-      const float worst = col[12 * ihi];
+      const float worst = comp ? col[12 * ihi] : 0.0f;
       const float pt = comp ? psum * fac1 - worst * fac2 : 0.0f;
       const float y = evaluate(pt);
       if (y < __shfl_sync(FULL, gv, ihi)) {
