@@ -33,7 +33,7 @@ struct VsgArgs {
   const int32_t* cell_off;   // [ncx * ncy + 1] into cell_pts / packed
   const int32_t* cell_pts;   // subset indices grouped by cell
   const int32_t* pos_of;     // position of each subset in cell order
-  const float2* centre;      // per position: x, y
+  float2* centre;            // per position: x, y as they are now
   float2* packed;            // per position: x (NaN when sigma < 0), y
   double2* packed_uv;        // per position: u, v as floats, widened
   int ncx, ncy;
@@ -51,8 +51,9 @@ __global__ void __launch_bounds__(256) vsg_pack_kernel(VsgArgs a) {
     const double* f = a.fields + (size_t)i * DICEGPU_FIELD_STRIDE;
     const bool valid = (float)f[DICEGPU_F_SIGMA] >= 0.0f;
     const int p = a.pos_of[i];
-    a.packed[p] = make_float2(valid ? (float)f[DICEGPU_F_COORD_X] : __int_as_float(0x7fc00000),
-                              (float)f[DICEGPU_F_COORD_Y]);
+    const float x = (float)f[DICEGPU_F_COORD_X], y = (float)f[DICEGPU_F_COORD_Y];
+    a.centre[p] = make_float2(x, y);
+    a.packed[p] = make_float2(valid ? x : __int_as_float(0x7fc00000), y);
     a.packed_uv[p] = make_double2((double)(float)f[DICEGPU_F_DISP_X], (double)(float)f[DICEGPU_F_DISP_Y]);
   }
 }
@@ -111,7 +112,9 @@ __global__ void __launch_bounds__(128) vsg_kernel(VsgArgs a) {
   const float2 ci = a.centre[t0];
   const float xi = ci.x, yi = ci.y;
   const bool self = !isnan(a.packed[t0].x);
-  const int gx = (int)floorf((xi - a.x0) / a.cell), gy = (int)floorf((yi - a.y0) / a.cell);
+  // the centre may have moved since the grid was built (dicegpu_fields_device_ptr)
+  const int gx = min(max((int)floorf((xi - a.x0) / a.cell), 0), a.ncx - 1);
+  const int gy = min(max((int)floorf((yi - a.y0) / a.cell), 0), a.ncy - 1);
   // sums: dx, dy, dx dx, dx dy, dy dy, u, dx u, dy u, v, dx v, dy v
   double s[11];
 #pragma unroll

@@ -1191,21 +1191,18 @@ static int build_vsg_grid(dicegpu_ctx* c, int window) {
   }
   for (size_t k = 0; k + 1 < off.size(); ++k) off[k + 1] += off[k];
   std::vector<int32_t> pos(n);
-  std::vector<float2> centre(n);
   {
     std::vector<int32_t> fill(off.begin(), off.end() - 1);
     for (int i = 0; i < n; ++i) {
       const int p = fill[cell_of[i]]++;
       pos[i] = p;
       pts[p] = i;
-      centre[p] = make_float2((float)coords[2 * (size_t)i], (float)coords[2 * (size_t)i + 1]);
     }
   }
   if ((rc = c->d_vsg_cell_off.ensure(off.size()))) return rc;
   CK(cudaMemcpy(c->d_vsg_cell_off.p, off.data(), off.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_vsg_cell_pts.p, pts.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_vsg_pos.p, pos.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_vsg_centre.p, centre.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
   c->h_vsg_coords.swap(coords);
   c->vsg_ncx = ncx;
   c->vsg_ncy = ncy;

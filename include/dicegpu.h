@@ -431,7 +431,10 @@ int dicegpu_get_uncertainty(dicegpu_ctx* ctx, double* out);
 /* Number of subsets of the context (0 before dicegpu_set_subsets). */
 int dicegpu_num_subsets(dicegpu_ctx* ctx, int* n);
 
-/* Device pointer of the field array (n * DICEGPU_FIELD_STRIDE doubles). */
+/* Device pointer of the field array (n * DICEGPU_FIELD_STRIDE doubles).
+ * dicegpu_vsg_strain reads the coordinates there at every call, but keeps its
+ * neighbour grid: after moving a centre by more than one pixel through this
+ * pointer, reload the fields (dicegpu_load_fields), which renews the grid. */
 int dicegpu_fields_device_ptr(dicegpu_ctx* ctx, double** dptr);
 /* Asynchronous copies of the whole field array on the context's stream
  * (`on_device` = 1 for device memory, 0 for host memory; pinned host memory
