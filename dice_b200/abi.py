@@ -31,6 +31,7 @@ BILINEAR, BICUBIC, KEYS_FOURTH = 0, 1, 2
 SIMPLEX, GRADIENT_BASED, SIMPLEX_THEN_GRADIENT_BASED, GRADIENT_BASED_THEN_SIMPLEX = 0, 1, 3, 4
 AFFINE_SF, QUADRATIC_SF = 0, 1
 FINITE_DIFFERENCE, CONVOLUTION_5_POINT = 0, 1
+STORAGE_ROWS, STORAGE_LEAN, STORAGE_SCRATCH = 0, 1, 2
 
 # ---- field columns ----------------------------------------------------------
 FIELD_STRIDE = 32
@@ -283,6 +284,8 @@ def _declare(lib):
                                      ctypes.POINTER(ctypes.c_float)]),
         "dicegpu_set_launch_shape": (c_int, [c_void_p, c_int, c_int]),
         "dicegpu_get_launch_shape": (c_int, [c_void_p, ctypes.POINTER(c_int), ctypes.POINTER(c_int)]),
+        "dicegpu_get_frame_launch": (c_int, [c_void_p, ctypes.POINTER(c_int), ctypes.POINTER(c_int),
+                                             ctypes.POINTER(c_int)]),
         "dicegpu_correlate": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
                                       c_int, c_int, P, c_int]),
         "dicegpu_correlate_reset": (c_int, []),

@@ -196,6 +196,9 @@ struct dicegpu_ctx {
   const void* wide_fn = nullptr;
   size_t wide_smem = 0;
   int wide_per_sm = 0;
+  // the latest frame launch (dicegpu_get_frame_launch)
+  FrameKernelFn lean_fn = nullptr;   // the lean kernel, once lean_launch took it
+  int last_storage = -1, last_warps = 0, last_blocks = 0;
   int carveout = -1;     // preferred shared-memory carveout (percent), -1: driver default
   long long launches = 0;
   // captured frame sequence
@@ -1531,6 +1534,12 @@ static int launch_frame(dicegpu_ctx* c, FrameKernelFn fn, const FrameArgs& a, in
   fn<<<blocks, warps * 32, smem, c->stream>>>(a);
   CK(cudaGetLastError());
   c->launches += 1;
+  if (a.mode == MODE_CORRELATE) {
+    c->last_storage = a.pix_scratch ? DICEGPU_STORAGE_SCRATCH
+                      : fn == c->lean_fn ? DICEGPU_STORAGE_LEAN : DICEGPU_STORAGE_ROWS;
+    c->last_warps = warps;
+    c->last_blocks = blocks;
+  }
   return DICEGPU_OK;
 }
 
@@ -1707,13 +1716,17 @@ static void wide_launch(dicegpu_ctx* c, FrameKernelFn fn, long n, int* warps, in
   *smem = s;
 }
 
-// A frame of large affine subsets, whose residual rows leave an SM one or two
-// CTAs of four warps, runs on the lean kernel when that fits more of them (the
-// registers allow four).  The double sums are those of the four warps either
-// way.  Frames that go to eight-warp CTAs (wide_launch) and launch shapes the
-// caller chose keep the rows.
+// A frame of large affine subsets, whose residual rows leave an SM three CTAs
+// of four warps or fewer, runs on the lean kernel when that fits more of them
+// (the registers allow four).  The double sums are those of the four warps
+// either way.  Frames that go to eight-warp CTAs (wide_launch) and launch
+// shapes the caller chose keep the rows, and so do rows in the global scratch:
+// four CTAs per SM from there are faster than the one that lean storage fits
+// in shared memory (2048^2, 91 px 14.8 and 21.5 ms, 99 px 18.6 and 25.7, 111 px
+// 24.0 and 32.8; 99 px bicubic 20.7 and 28.4).
 static bool lean_launch(dicegpu_ctx* c, FrameKernelFn* fn, int* blocks, size_t* smem) {
-  if (c->dp.shape != DICEGPU_AFFINE_SF || c->use_masks || c->shape_set || c->n <= 6L * *blocks) return false;
+  if (c->dp.shape != DICEGPU_AFFINE_SF || c->use_masks || c->pix_in_global || c->shape_set || c->n <= 6L * *blocks)
+    return false;
   const int per_sm = *blocks / c->num_sms;
   if (per_sm > DG_LEAN_BELOW) return false;
   FrameKernelFn lf = pick_frame_kernel(kAffineLean, c->dp.interp, c->params.use_def_gradients != 0, false);
@@ -1727,8 +1740,8 @@ static bool lean_launch(dicegpu_ctx* c, FrameKernelFn* fn, int* blocks, size_t* 
     cudaGetLastError();
     return false;
   }
-  if (lean_sm <= per_sm && !c->pix_in_global) return false;
-  *fn = lf;
+  if (lean_sm <= per_sm) return false;
+  *fn = c->lean_fn = lf;
   *blocks = std::min(lean_sm * c->num_sms, kMaxGrid);
   *smem = s;
   return true;
@@ -1827,8 +1840,7 @@ extern "C" int dicegpu_execute_correlation(dicegpu_ctx* c) {
   FrameArgs a;
   fill_args(c, a, MODE_CORRELATE);
   int warps = c->warps_per_cta;
-  if (lean_launch(c, &fn, &blocks, &smem)) a.pix_scratch = nullptr;
-  else wide_launch(c, fn, c->n, &warps, &blocks, &smem);
+  if (!lean_launch(c, &fn, &blocks, &smem)) wide_launch(c, fn, c->n, &warps, &blocks, &smem);
   if ((rc = launch_frame(c, fn, a, c->n, blocks, warps, smem))) return rc;
   return frame_end(c);
 }
@@ -2073,6 +2085,15 @@ extern "C" int dicegpu_get_launch_shape(dicegpu_ctx* c, int* warps_per_cta, int*
   if (!c || !warps_per_cta || !ctas_per_sm) return DICEGPU_ERR_ARG;
   *warps_per_cta = c->warps_per_cta;
   *ctas_per_sm = c->ctas_per_sm;
+  return DICEGPU_OK;
+}
+
+extern "C" int dicegpu_get_frame_launch(dicegpu_ctx* c, int* storage, int* warps_per_cta, int* ctas) {
+  if (!c || !storage || !warps_per_cta || !ctas) return DICEGPU_ERR_ARG;
+  if (c->last_storage < 0) return DICEGPU_ERR_STATE;
+  *storage = c->last_storage;
+  *warps_per_cta = c->last_warps;
+  *ctas = c->last_blocks;
   return DICEGPU_OK;
 }
 

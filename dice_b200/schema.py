@@ -79,6 +79,13 @@ class Schema:
                   "get_launch_shape")
         return a.value, b.value
 
+    def frame_launch(self):
+        """(storage, warps per CTA, CTAs) of the latest frame kernel; storage: abi.STORAGE_*."""
+        s, w, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+        abi.check(self.lib.dicegpu_get_frame_launch(self.ctx, ctypes.byref(s), ctypes.byref(w), ctypes.byref(b)),
+                  "get_frame_launch")
+        return s.value, w.value, b.value
+
     # ---- images ---------------------------------------------------------------
     def _image_call(self, fn, img, what):
         # 8- and 16-bit images go through the typed entry points (converted on

@@ -488,6 +488,14 @@ int dicegpu_launch_count(dicegpu_ctx* ctx, int64_t* count);
 int dicegpu_set_launch_shape(dicegpu_ctx* ctx, int warps_per_cta, int ctas_per_sm);
 int dicegpu_get_launch_shape(dicegpu_ctx* ctx, int* warps_per_cta, int* ctas_per_sm);
 
+/* How the latest kernel of dicegpu_execute_correlation was launched: where a
+ * subset's per-pixel rows were kept, the warps per CTA, and the number of
+ * CTAs.  DICEGPU_ERR_STATE before the first one. */
+#define DICEGPU_STORAGE_ROWS    0   /* shared memory */
+#define DICEGPU_STORAGE_LEAN    1   /* shared memory, affine residuals formed again instead of stored */
+#define DICEGPU_STORAGE_SCRATCH 2   /* global memory: the rows exceed a CTA's shared memory */
+int dicegpu_get_frame_launch(dicegpu_ctx* ctx, int* storage, int* warps_per_cta, int* ctas);
+
 /* ---- stride-9 API (mirror of dice_correlate) ------------------------------
  * Replaces dice_correlate (DICe_api.cpp:51-151); update_params is its
  * `const bool update_params`.  points: n * 9 floats [x, y, u, v, theta,
