@@ -127,7 +127,7 @@ __global__ void interp_kernel(int method, int w, int h, const float* __restrict_
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
-// affine subsets are stored lean when their rows leave an SM this many CTAs or fewer
+// affine subsets can be stored lean when their rows leave an SM this many CTAs or fewer
 #ifndef DG_LEAN_BELOW
 #define DG_LEAN_BELOW 3
 #endif
@@ -1717,32 +1717,45 @@ static void wide_launch(dicegpu_ctx* c, FrameKernelFn fn, long n, int* warps, in
 }
 
 // A frame of large affine subsets, whose residual rows leave an SM three CTAs
-// of four warps or fewer, runs on the lean kernel when that fits more of them
-// (the registers allow four).  The double sums are those of the four warps
-// either way.  Frames that go to eight-warp CTAs (wide_launch) and launch
-// shapes the caller chose keep the rows, and so do rows in the global scratch:
-// four CTAs per SM from there are faster than the one that lean storage fits
-// in shared memory (2048^2, 91 px 14.8 and 21.5 ms, 99 px 18.6 and 25.7, 111 px
-// 24.0 and 32.8; 99 px bicubic 20.7 and 28.4).
+// or fewer, runs on the lean kernel when that fits more of them (registers
+// allow four of four warps).  The double sums are those of the same warps
+// either way.  This is a choice of storage: it is made for the launch shape in
+// force, whether the caller, the autotuner or the default set it.  Rows and
+// lean, ms per frame of 2048^2 at 1, 2, 4 and 8 warps:
+//   41 px  21.4 13.0, 13.7 9.8, 9.2 8.3, 10.3 10.7 (two CTAs either way: rows kept)
+//   61 px  41.7 18.4, 24.3 11.5, 13.8 7.1, 10.9 7.0
+//   71 px  39.9 22.7, 22.8 13.7, 12.7 8.1, 9.6 6.3
+//   81 px  52.4 30.8, 29.6 32.6 (one CTA either way: rows kept), 16.4 17.5, 12.1 12.6
+// Frames that go to eight-warp CTAs (wide_launch) keep the rows, and so do rows
+// in the global scratch: four CTAs per SM from there are faster than the one
+// that lean storage fits in shared memory (91 px 14.8 and 21.5 ms, 99 px 18.6
+// and 25.7, 111 px 24.0 and 32.8; 99 px bicubic 20.7 and 28.4).
 static bool lean_launch(dicegpu_ctx* c, FrameKernelFn* fn, int* blocks, size_t* smem) {
-  if (c->dp.shape != DICEGPU_AFFINE_SF || c->use_masks || c->pix_in_global || c->shape_set || c->n <= 6L * *blocks)
-    return false;
-  const int per_sm = *blocks / c->num_sms;
-  if (per_sm > DG_LEAN_BELOW) return false;
+  if (c->dp.shape != DICEGPU_AFFINE_SF || c->use_masks || c->pix_in_global) return false;
+  const int threads = c->warps_per_cta * 32, asked = c->ctas_per_sm;
+  int rows_sm = *blocks / c->num_sms, lean_sm = 0;   // resident CTAs
+  if (asked > 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rows_sm, (const void*)*fn, threads, *smem) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    rows_sm = std::min(rows_sm, asked);
+  }
+  if (rows_sm > DG_LEAN_BELOW || c->n <= 6L * rows_sm * c->num_sms) return false;
   FrameKernelFn lf = pick_frame_kernel(kAffineLean, c->dp.interp, c->params.use_def_gradients != 0, false);
   size_t fixed, pix;
   frame_smem_bytes(c, c->warps_per_cta, &fixed, &pix, true);
   const size_t s = fixed + pix;
   if (!lf || s > (size_t)c->smem_optin) return false;
-  int lean_sm = 0;
   if (cudaFuncSetAttribute((const void*)lf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lean_sm, (const void*)lf, c->warps_per_cta * 32, s) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lean_sm, (const void*)lf, threads, s) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  if (lean_sm <= per_sm) return false;
+  if (asked > 0) lean_sm = std::min(lean_sm, asked);
+  if (lean_sm <= rows_sm) return false;
   *fn = c->lean_fn = lf;
-  *blocks = std::min(lean_sm * c->num_sms, kMaxGrid);
+  *blocks = std::min((asked > 0 ? asked : lean_sm) * c->num_sms, kMaxGrid);
   *smem = s;
   return true;
 }

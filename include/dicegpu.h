@@ -484,7 +484,8 @@ int dicegpu_launch_count(dicegpu_ctx* ctx, int64_t* count);
  * keeps the current value.  Until a shape is set here or by
  * dicegpu_autotune, a launch with at most six subsets per default-shape CTA
  * (small tracking waves, small frames, per-subset launches) and a chain of
- * single-subset waves run on CTAs of eight warps. */
+ * single-subset waves run on CTAs of eight warps.  Where a subset's rows are
+ * kept is decided for the shape in force, whoever set it. */
 int dicegpu_set_launch_shape(dicegpu_ctx* ctx, int warps_per_cta, int ctas_per_sm);
 int dicegpu_get_launch_shape(dicegpu_ctx* ctx, int* warps_per_cta, int* ctas_per_sm);
 

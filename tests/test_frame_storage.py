@@ -2,6 +2,7 @@
 while they leave an SM four CTAs, lean where that fits more CTAs, the rows
 again where one CTA fits either way, global scratch beyond a CTA's shared
 memory."""
+import numpy as np
 import pytest
 
 from dice_b200 import abi
@@ -35,3 +36,41 @@ def test_storage_by_subset_size(subset, step, storage):
             s.frame_launch()   # none yet
         s.execute_correlation()
         assert s.frame_launch()[:2] == (storage, 4)
+
+
+def test_storage_does_not_depend_on_who_set_the_launch_shape():
+    """61 px: one CTA per SM with rows, three of four warps lean."""
+    with _schema(61, 10) as s:
+        f = s.fields()
+        s.execute_correlation()
+        want = s.fields()
+        assert s.frame_launch()[:2] == (abi.STORAGE_LEAN, 4)
+        ctas = s.frame_launch()[2]
+        for shape, storage, grid in [((4, 0), abi.STORAGE_LEAN, ctas), ((4, 1), abi.STORAGE_ROWS, ctas // 3),
+                                     ((4, 2), abi.STORAGE_LEAN, ctas // 3 * 2), ((8, 0), abi.STORAGE_LEAN, None),
+                                     ((2, 0), abi.STORAGE_LEAN, None), ((1, 0), abi.STORAGE_LEAN, None)]:
+            # a context of its own: 0 CTAs per SM keeps an earlier value
+            with _schema(61, 10) as t:
+                t.set_launch_shape(*shape)
+                t.execute_correlation()
+                assert t.frame_launch()[:2] == (storage, shape[0])
+                assert grid is None or t.frame_launch()[2] == grid
+                got = t.fields()
+            if shape[0] == 4:
+                assert np.array_equal(got, want)   # the same warps: the same sums
+            else:
+                # a shape may move a double sum's last bit, and a float of the
+                # parameters (below 16) with it, before the last iterations
+                ok = want[:, abi.F_SIGMA] >= 0
+                assert ok.mean() > 0.9
+                uv = slice(abi.F_DISP_X, abi.F_DISP_Y + 1)
+                assert np.abs(got[ok, uv] - want[ok, uv]).max() < 1e-4
+        s.load_fields(f)
+        s.autotune()
+        s.load_fields(f)
+        s.execute_correlation()
+        assert s.frame_launch()[0] == abi.STORAGE_LEAN
+    with _schema(61, 10) as s:   # the tuner's cache
+        s.autotune()
+        s.execute_correlation()
+        assert s.frame_launch()[0] == abi.STORAGE_LEAN
