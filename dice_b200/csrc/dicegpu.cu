@@ -576,16 +576,27 @@ static bool gauss_weights(int M, GaussWeights& g) {
   return true;
 }
 
-static int launch_gauss_filter(int w, int h, int M, const float* in, float* out, cudaStream_t st,
+// the current device's multiprocessors
+static int device_sms(int* sms) {
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
+  return DICEGPU_OK;
+}
+
+// sms: the device's multiprocessors, 0 to ask for them
+static int launch_gauss_filter(int w, int h, int M, const float* in, float* out, cudaStream_t st, int sms,
                                long long* launches) {
   GaussWeights g;
   if (!gauss_weights(M, g)) return DICEGPU_ERR_ARG;
   if (w < M || h < M) return DICEGPU_ERR_ARG;
+  int rc;
+  if (sms < 1 && (rc = device_sms(&sms))) return rc;
   // Eight rows a thread while that leaves every SM two CTAs, else two.  Eight
-  // and two rows: 2048^2 22.9 and 25.1 us at M = 7, 52.4 and 57.8 at M = 13; 512^2
+  // and two rows on 148 SMs: 2048^2 22.9 and 25.1 us at M = 7, 52.4 and 57.8 at M = 13; 512^2
   // (64 CTAs with eight) 8.3 and 8.0, 12.8 and 8.6; 1024^2 10.7 and 8.7, 18.9 and 18.8.
   const unsigned gx = (w + 2 * kGaussBX - 1) / (2 * kGaussBX);
-  const bool tall = (long long)gx * ((h + 8 * kGaussBY - 1) / (8 * kGaussBY)) >= 2 * 148;
+  const bool tall = (long long)gx * ((h + 8 * kGaussBY - 1) / (8 * kGaussBY)) >= 2LL * sms;
   const unsigned rows = kGaussBY * (tall ? 8 : 2);
   const dim3 blk(kGaussBX, kGaussBY), grd(gx, (h + rows - 1) / rows);
   void (*fn)(int, int, GaussWeights, f32x2, const float*, float*) = nullptr;
@@ -612,7 +623,7 @@ static int upload_image(dicegpu_ctx* c, float* dst, const float* src, int on_dev
       CK(cudaMemcpyAsync(c->d_tmp, src, bytes, cudaMemcpyHostToDevice, c->stream));
       raw = c->d_tmp;
     }
-    return launch_gauss_filter(c->W, c->H, c->params.gauss_filter_mask_size, raw, dst, c->stream,
+    return launch_gauss_filter(c->W, c->H, c->params.gauss_filter_mask_size, raw, dst, c->stream, c->num_sms,
                                &c->launches);
   }
   CK(cudaMemcpyAsync(dst, src, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
@@ -650,7 +661,7 @@ static int upload_typed(dicegpu_ctx* c, float* dst, const void* src, int type, i
   CK(cudaGetLastError());
   c->launches += 1;
   if (c->params.gauss_filter_images)
-    return launch_gauss_filter(c->W, c->H, c->params.gauss_filter_mask_size, conv, dst, c->stream,
+    return launch_gauss_filter(c->W, c->H, c->params.gauss_filter_mask_size, conv, dst, c->stream, c->num_sms,
                                &c->launches);
   return DICEGPU_OK;
 }
@@ -2340,7 +2351,7 @@ extern "C" int dicegpu_image_gradients(int w, int h, const float* d_img, float* 
 extern "C" int dicegpu_gauss_filter(int w, int h, const float* d_in, float* d_out, int mask_size,
                                     void* stream) {
   if (!d_in || !d_out || d_in == d_out || w < 1 || h < 1) return DICEGPU_ERR_ARG;
-  return launch_gauss_filter(w, h, mask_size, d_in, d_out, (cudaStream_t)stream, nullptr);
+  return launch_gauss_filter(w, h, mask_size, d_in, d_out, (cudaStream_t)stream, 0, nullptr);
 }
 
 // ---------------------------------------------------------------------------
