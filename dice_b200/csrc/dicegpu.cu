@@ -2363,9 +2363,9 @@ extern "C" int dicegpu_gauss_filter(int w, int h, const float* d_in, float* d_ou
 // for the whole device).  The copy that dicegpu_image_gradients allocates
 // when the 5-point smoothing writes over its own input lives instead in the
 // file-scope array below, which every GPU that loads this library holds until
-// the process exits (8 MiB).
+// the process exits (4 MiB).
 // ---------------------------------------------------------------------------
-static __device__ __align__(256) float g_noalloc_scratch[2 * DICEGPU_NOALLOC_MAX_PIXELS];
+static __device__ __align__(256) float g_noalloc_scratch[DICEGPU_NOALLOC_MAX_PIXELS];
 
 namespace {
 constexpr int kMaxDevices = 64;

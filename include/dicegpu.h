@@ -553,7 +553,7 @@ int dicegpu_gauss_filter(int w, int h, const float* d_in, float* d_out, int mask
  * their own pool or budget, and per-frame loops that cannot afford the
  * device-wide wait of cudaFree.  When the smoothing writes over its own
  * input (d_gx or d_gy overlaps d_img), the input is first copied to a
- * file-scope device array of 2 * DICEGPU_NOALLOC_MAX_PIXELS floats (8 MiB)
+ * file-scope device array of DICEGPU_NOALLOC_MAX_PIXELS floats (4 MiB)
  * that every GPU loading the library holds until exit.
  * With DICEGPU_CONVOLUTION_5_POINT, images larger than
  * DICEGPU_NOALLOC_MAX_PIXELS pixels are rejected with DICEGPU_ERR_ARG;
