@@ -260,7 +260,8 @@ __device__ void adjoint_subset(const AdjointArgs& A, int idx) {
 // subset): 6 taps are loaded and 6 sums go to the image per pixel instead of
 // 36 and 36.  (A pixel per lane in reading order, 36 loads and 36 atomics: 657 us
 // for 19,600 25 x 25 subsets, bound by the L1's wavefronts; the operations
-// per value are the same.)
+// per value are the same.)  Subsets far from a translation, whose windows seldom
+// slide, are left to adjoint_distorted_kernel.
 template <int SHAPE>
 struct AdjointColumn {
   const AdjointArgs& A;
@@ -332,6 +333,18 @@ struct AdjointColumn {
   }
 };
 
+// Whether the magnitudes of the displacement's gradients (at the centre) add
+// up to more than 0.34.  Columns and pixels, us for 19,600 25 px subsets: sum 0.
+// 597 and 670; 0.23 962 and 980; 0.33 815 and 815; 0.35 1,035 and 940; 0.46 1,362
+// and 1,160; rotations of 0.4, 0.79 and 1.57 rad 1,718 and 1,435, 2,625 and
+// 2,180, 4,940 and 4,030.  (15 px, 0.79 rad: 1,370 and 930.)
+template <int SHAPE>
+__device__ __forceinline__ bool adjoint_distorted(const float* s) {
+  const float sum = SHAPE == DICEGPU_QUADRATIC_SF ? fabsf(s[0] - 1.0f) + fabsf(s[1]) + fabsf(s[6]) + fabsf(s[7] - 1.0f)
+                                                  : 2.0f * fmaxf(fabsf(s[2]), fabsf(s[5])) + fabsf(s[3]) + fabsf(s[4]);
+  return !(sum <= 0.34f);
+}
+
 template <int SHAPE>
 __device__ void adjoint_square(const AdjointArgs& A, int idx) {
   const double* f = A.fields + (size_t)idx * DICEGPU_FIELD_STRIDE;
@@ -341,10 +354,14 @@ __device__ void adjoint_square(const AdjointArgs& A, int idx) {
   adjoint_slots<SHAPE>(f, slots);
   MapConst k;
   make_mapconst<SHAPE>(slots, false, fcx, fcy, k);
+  const bool distorted = adjoint_distorted<SHAPE>(slots);
   AdjointColumn<SHAPE> c(A, k, cx, cy);
   const long rlim = (long)A.ref.w * A.ref.h;
   // pass 1: moments over the active pixels
   double n = 0.0, sF = 0.0, sF2 = 0.0, sG = 0.0, sG2 = 0.0, sGF = 0.0;
+  // (left here, after the map's constants: before them it costs 4 us of 598,
+  // the field row's loads no longer overlapping)
+  if (distorted) return;
 #pragma unroll 1
   for (int chunk = 0; chunk < c.chunks(); ++chunk) {
     c.start(chunk);
@@ -491,6 +508,28 @@ __global__ void __launch_bounds__(256) adjoint_kernel(const __grid_constant__ Ad
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; idx < a.n; idx += warps)
     adjoint_subset<SHAPE>(a, idx);
+}
+
+// The squares that adjoint_square leaves, a pixel per lane: lane l of a warp
+// looks at the warp's l-th next subset, and the warp takes those found.  A
+// launch of its own (3 us when there are none): with both paths in one kernel,
+// the columns lose 10 us of 598.
+template <int SHAPE>
+__global__ void __launch_bounds__(256) adjoint_distorted_kernel(const __grid_constant__ AdjointArgs a) {
+  const int warps = (gridDim.x * blockDim.x) >> 5, lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (long long first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; first < a.n; first += 32LL * warps) {
+    const long long mine = first + (long long)lane * warps;
+    bool distorted = false;
+    if (mine < a.n) {
+      float slots[12];
+      adjoint_slots<SHAPE>(a.fields + (size_t)mine * DICEGPU_FIELD_STRIDE, slots);
+      distorted = adjoint_distorted<SHAPE>(slots);
+    }
+#pragma unroll 1
+    for (unsigned left = __ballot_sync(FULL, distorted); left; left &= left - 1)
+      adjoint_subset<SHAPE>(a, (int)first + (__ffs(left) - 1) * warps);
+  }
 }
 
 }  // namespace dg

@@ -2274,15 +2274,20 @@ extern "C" int dicegpu_adjoint(dicegpu_ctx* c, const double* d_fields, const dou
   void (*fn)(AdjointArgs);
   if (columns) fn = quad ? adjoint_square_kernel<DICEGPU_QUADRATIC_SF> : adjoint_square_kernel<DICEGPU_AFFINE_SF>;
   else fn = quad ? adjoint_kernel<DICEGPU_QUADRATIC_SF> : adjoint_kernel<DICEGPU_AFFINE_SF>;
-  const int threads = columns ? 128 : 256;
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, threads, 0));
-  const int need = (c->n + threads / 32 - 1) / (threads / 32);
-  const int blocks = std::max(1, std::min(std::max(per_sm, 1) * c->num_sms, need));
-  fn<<<blocks, threads, 0, c->stream>>>(a);
-  CK(cudaGetLastError());
-  c->launches += 1;
-  return DICEGPU_OK;
+  auto launch = [&](void (*f)(AdjointArgs), int threads) -> int {
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)f, threads, 0));
+    const int need = (c->n + threads / 32 - 1) / (threads / 32);
+    const int blocks = std::max(1, std::min(std::max(per_sm, 1) * c->num_sms, need));
+    f<<<blocks, threads, 0, c->stream>>>(a);
+    CK(cudaGetLastError());
+    c->launches += 1;
+    return DICEGPU_OK;
+  };
+  rc = launch(fn, columns ? 128 : 256);
+  if (!rc && columns)
+    rc = launch(quad ? adjoint_distorted_kernel<DICEGPU_QUADRATIC_SF> : adjoint_distorted_kernel<DICEGPU_AFFINE_SF>, 256);
+  return rc;
 }
 
 extern "C" int dicegpu_interpolate(dicegpu_ctx* c, int method, int n, const float* xy,
