@@ -533,14 +533,20 @@ int dicegpu_correlate_reset(void);
 int dicegpu_interpolate(dicegpu_ctx* ctx, int method, int n, const float* xy,
                         float* intensity, float* grad_x, float* grad_y, int on_device);
 
-/* Finite-difference gradients of a float image (both device pointers).
+/* Finite-difference gradients of a float image (device pointers), smoothed
+ * with DICEGPU_CONVOLUTION_5_POINT.  Ordered on `stream` and asynchronous:
+ * d_gx and d_gy hold the gradients, and d_img may be overwritten, once the
+ * stream's work is done.  Only a smoothing that writes over its own input
+ * (d_gx or d_gy overlaps d_img) copies the image to memory that it allocates,
+ * and waits for the stream before it returns.
  * Replaces Image_::compute_gradients (DICe_Image.cpp:1015-1093). */
 int dicegpu_image_gradients(int w, int h, const float* d_img, float* d_gx, float* d_gy,
                             int method, void* stream);
 
 /* Gaussian filter of a float image with a mask_size x mask_size mask (5, 7,
  * 9, 11 or 13); pixels closer than mask_size/2+1 to an edge keep their
- * value.  d_in and d_out are device pointers to different buffers.
+ * value.  d_in and d_out are device pointers to different buffers.  Ordered
+ * on `stream` and asynchronous.
  * Replaces Image_::gauss_filter (DICe_Image.cpp:1194-1230).  Images smaller
  * than the mask are rejected with DICEGPU_ERR_ARG, as the reference
  * throws. */
