@@ -50,7 +50,7 @@ static __device__ unsigned long long g_prof[16];   // per translation unit
 #endif
 
 // An affine subset stored lean: 17 bytes per pixel instead of 33.  For subsets
-// so large that their residual rows leave an SM one or two CTAs.
+// so large that their residual rows leave an SM three CTAs or fewer.
 constexpr int kAffineLean = 2;
 
 template <int SHAPE>
