@@ -185,8 +185,8 @@ def cpu_sample(p, ref, frames, n_sample, nthreads, timed_frames=1, uncertainty=F
 SIMPLEX_FLOP_PER_PIXEL_EVAL = 200.0
 # DRAM bytes (read + write) of one frame_kernel launch of the full frame
 # (158,404 subsets, a frame of the sequence), from an ncu capture of that
-# launch: dram__bytes_read.sum 157.6 MB + dram__bytes_write.sum 38.2 MB
-FRAME_KERNEL_DRAM_BYTES = 157.641e6 + 38.175e6
+# launch: dram__bytes_read.sum 144.0 MB + dram__bytes_write.sum 22.7 MB
+FRAME_KERNEL_DRAM_BYTES = 143.999e6 + 22.716e6
 
 
 def oracle_sequence_sample(p, ref_h, frames_h, stride, nthreads, uncertainty=False, library=None):
@@ -688,8 +688,8 @@ def run_adjoint(args):
                "l2": "flushed between timed steps (256 MiB write)", "parallelism": "replicas x%d" % world}
         roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak if peak else None, "traffic": None,
-                "per_unit": "%d FP32 flop per subset pixel (both passes) plus 36 atomic adds" % ADJ_FLOP_PER_PIXEL,
-                "kernel": "adjoint_kernel (median step incl. clearing the image derivative)"}
+                "per_unit": "%d FP32 flop per subset pixel (both passes) plus 6 atomic adds" % ADJ_FLOP_PER_PIXEL,
+                "kernel": "adjoint_square_kernel (median step incl. clearing the image derivative)"}
         print(json.dumps(_line("subset objective adjoints/sec (value, d/dparams, d/dimage)", value, "subsets/s",
                                world, args, total_ms / args.steps, cfg, roofline=roof,
                                cpu_baseline={"value": None, "note": "the reference has no derivative code"},
@@ -1247,10 +1247,11 @@ def main():
             "frac": fp32_tflops / fp32_peak if (fp32_peak and fp32_tflops) else None,
             "traffic": FRAME_KERNEL_DRAM_BYTES,
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one frame_kernel launch "
-                              "on a full frame (reads 157.6 MB, writes 38.2 MB)",
-            "issue": {"inst_per_cycle_per_scheduler": 0.43, "warp_instructions_per_frame": 28.9e9,
-                      "source": "ncu smsp__issue_active / smsp__inst_executed.sum of the same capture; the "
-                                "binding resource is instruction issue, not a math pipe or DRAM"},
+                              "on a full frame (reads 144.0 MB, writes 22.7 MB)",
+            "issue": {"inst_per_cycle_per_scheduler": 0.50, "warp_instructions_per_frame": 28.0e9,
+                      "source": "ncu smsp__issue_active / smsp__inst_executed.sum of the same capture; what "
+                                "binds is latency at 16 warps per SM (barriers behind the serial sums and "
+                                "the solve, FP64 and conversion results, taps), not a math pipe or DRAM"},
             "kernel": "frame_kernel (median step time incl. the gradient and pack kernels)",
             "peak_source": "measured FP32 SGEMM on CUDA cores (TF32 off) in this run",
             "per_unit": "390 FP32 flop per active pixel per Gauss-Newton pass + 200 per simplex evaluation, "
