@@ -1510,6 +1510,13 @@ static void fill_args(dicegpu_ctx* c, FrameArgs& a, int mode) {
   a.unc = (c->params.compute_uncertainty && c->unc_n == c->n) ? c->d_unc : nullptr;
 }
 
+// The limit of a kernel's dynamic shared memory belongs to the process: every
+// context sets it to the device's, so that one thread's frames never lower it
+// under another's (a launch takes what it asks for, whatever the limit).
+static cudaError_t allow_smem(const dicegpu_ctx* c, FrameKernelFn fn) {
+  return cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin);
+}
+
 static int grid_for(dicegpu_ctx* c, FrameKernelFn fn, int* blocks, size_t* smem) {
   if (!fn) return DICEGPU_ERR_UNSUPPORTED;
   const int threads = c->warps_per_cta * 32;
@@ -1520,7 +1527,7 @@ static int grid_for(dicegpu_ctx* c, FrameKernelFn fn, int* blocks, size_t* smem)
   c->pix_in_global = fixed + pix > (size_t)c->smem_optin;
   *smem = c->pix_in_global ? fixed : fixed + pix;
   c->pix_stride = pix;
-  CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+  CK(allow_smem(c, fn));
   if (c->carveout >= 0)
     CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout, c->carveout));
   int per_sm = c->ctas_per_sm;
@@ -1689,9 +1696,6 @@ static void chain_shape(dicegpu_ctx* c, FrameKernelFn fn, int* warps, size_t* sm
   frame_smem_bytes(c, w, &fixed, &pix);
   const size_t s = c->pix_in_global ? fixed : fixed + pix;
   if (s > (size_t)c->smem_optin) return;
-  if (s > *smem &&
-      cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s) != cudaSuccess)
-    return;
   *warps = w;
   *smem = s;
 }
@@ -1709,9 +1713,6 @@ static void wide_launch(dicegpu_ctx* c, FrameKernelFn fn, long n, int* warps, in
   frame_smem_bytes(c, w, &fixed, &pix);
   const size_t s = c->pix_in_global ? fixed : fixed + pix;
   if (s > (size_t)c->smem_optin) return;
-  if (s > *smem &&
-      cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s) != cudaSuccess)
-    return;
   if (c->wide_fn != (const void*)fn || c->wide_smem != s) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, w * 32, s) != cudaSuccess)
@@ -1758,7 +1759,7 @@ static bool lean_launch(dicegpu_ctx* c, FrameKernelFn* fn, int* blocks, size_t* 
   frame_smem_bytes(c, c->warps_per_cta, &fixed, &pix, true);
   const size_t s = fixed + pix;
   if (!lf || s > (size_t)c->smem_optin) return false;
-  if (cudaFuncSetAttribute((const void*)lf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s) != cudaSuccess ||
+  if (allow_smem(c, lf) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lean_sm, (const void*)lf, threads, s) != cudaSuccess) {
     cudaGetLastError();
     return false;
