@@ -74,3 +74,22 @@ def test_storage_does_not_depend_on_who_set_the_launch_shape():
         s.autotune()
         s.execute_correlation()
         assert s.frame_launch()[0] == abi.STORAGE_LEAN
+
+
+def test_lean_frames_in_a_captured_sequence():
+    torch = pytest.importorskip("torch")
+    with _schema(61, 10) as s:
+        f = s.fields()
+        s.execute_correlation()
+        want = s.fields()
+    frame = syn.warp_image(syn.speckle_image(640, 640, seed=640, blur_sigma=0.8),
+                           lambda X, Y: (0.3 + 0.002 * X, -0.2 + 0.001 * Y), noise_sigma=1.0, seed=3, clip=(0.0, 255.0)).cuda()
+    with _schema(61, 10) as g:
+        g.set_stream(torch.cuda.Stream())
+        reset = torch.from_numpy(f).cuda()
+        torch.cuda.synchronize()
+        g.capture_sequence([frame], reset_fields=reset)
+        assert g.frame_launch()[:2] == (abi.STORAGE_LEAN, 4)
+        for _ in range(2):
+            g.launch_sequence()
+            assert np.array_equal(g.fields(), want)
