@@ -656,8 +656,8 @@ struct Engine {
   // its own copy, so that all take the same branches and evaluate the same
   // points together.  Lane j holds component j of the points and sums (the
   // vertices in the warp's SimplexState, where it alone reads and writes its
-  // column; lanes without a component touch none), lane i the value at vertex i; what all lanes need comes by
-  // shuffles.  (With every thread keeping all components, the bookkeeping took
+  // column; lanes without a component touch none), lane i the value at vertex
+  // i; what all lanes need comes by shuffles.  (With every thread keeping all components, the bookkeeping took
   // 30 % of a simplex subset's time.)  `slots` in/out: left at the last
   // evaluated point, as the reference's aliasing of variables and
   // shape-function parameters leaves it (DICe_LocalShapeFunction.h:259-261).

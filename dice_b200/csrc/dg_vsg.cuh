@@ -19,7 +19,10 @@
 // pivoting and an explicit inverse (the reference's GETRF / GETRI).  The sums
 // are exact for the reference's integer centres unless displacements span more
 // than about 2^9, so their order does not show.  (With a warp per subset
-// at a time, twelve warp-wide double sums each, 158,404 subsets took 265 us.)
+// at a time, twelve warp-wide double sums each, 158,404 subsets took 265 us, now
+// 75.  A thread waits for one candidate after the other, which shows with few
+// subsets and very many neighbours: 2,500 subsets with 1,250 neighbours each 232
+// us against 198.)
 // The condition number is computed exactly where the reference estimates it
 // (GECON); the two differ only for nearly collinear neighbourhoods.
 #pragma once

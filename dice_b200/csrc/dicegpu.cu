@@ -1738,10 +1738,14 @@ static void wide_launch(dicegpu_ctx* c, FrameKernelFn fn, long n, int* warps, in
 //   61 px  41.7 18.4, 24.3 11.5, 13.8 7.1, 10.9 7.0
 //   71 px  39.9 22.7, 22.8 13.7, 12.7 8.1, 9.6 6.3
 //   81 px  52.4 30.8, 29.6 32.6 (one CTA either way: rows kept), 16.4 17.5, 12.1 12.6
-// Frames that go to eight-warp CTAs (wide_launch) keep the rows, and so do rows
-// in the global scratch: four CTAs per SM from there are faster than the one
-// that lean storage fits in shared memory (91 px 14.8 and 21.5 ms, 99 px 18.6
-// and 25.7, 111 px 24.0 and 32.8; 99 px bicubic 20.7 and 28.4).
+// Frames of at most six subsets per CTA of the rows' grid, which eight-warp CTAs
+// take (wide_launch), keep the rows: a subset alone is faster with them (61 px
+// at eight warps, 140 subsets 210 and 227 us).  From the second subset per CTA
+// on, lean would gain there too (400 subsets 553 and 471 us, 800 1,035 and 706):
+// the two choices are not combined.  Rows in the global scratch stay there: four
+// CTAs per SM are faster than the one that lean storage fits in shared memory
+// (91 px 14.8 and 21.5 ms, 99 px 18.6 and 25.7, 111 px 24.0 and 32.8; 99 px
+// bicubic 20.7 and 28.4).
 static bool lean_launch(dicegpu_ctx* c, FrameKernelFn* fn, int* blocks, size_t* smem) {
   if (c->dp.shape != DICEGPU_AFFINE_SF || c->use_masks || c->pix_in_global) return false;
   const int threads = c->warps_per_cta * 32, asked = c->ctas_per_sm;
