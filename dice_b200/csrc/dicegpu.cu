@@ -496,6 +496,15 @@ extern "C" int dicegpu_set_stream(dicegpu_ctx* c, void* stream) {
   return DICEGPU_OK;
 }
 
+// Host memory to the device, done when it returns.  On the context's stream,
+// not by cudaMemcpy: from pageable memory that returns with the last part
+// still on its way, ordered on the legacy stream only, and a kernel on a
+// non-blocking stream may read ahead of it.
+static cudaError_t upload(dicegpu_ctx* c, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
 static int ensure_images(dicegpu_ctx* c, int w, int h) {
   const size_t npx = (size_t)w * h;
   if (c->has_ref && (c->W != w || c->H != h)) {
@@ -727,7 +736,7 @@ extern "C" int dicegpu_set_neighbors(dicegpu_ctx* c, const int32_t* neighbor_ids
   cudaStreamSynchronize(c->stream);
   int rc = c->d_neigh.ensure(n);
   if (rc) return rc;
-  CK(cudaMemcpy(c->d_neigh.p, nb.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_neigh.p, nb.data(), n * sizeof(int32_t)));
   c->h_neigh.swap(nb);
   return DICEGPU_OK;
 }
@@ -792,10 +801,10 @@ extern "C" int dicegpu_set_subset_pixels(dicegpu_ctx* c, int n, const int32_t* o
   if ((rc = grow(&c->d_px, &c->list_cap, total))) return rc;
   if ((rc = grow(&c->d_py, &cap2, total))) return rc;
   c->list_cap = std::min(c->list_cap, cap2);
-  CK(cudaMemcpy(c->d_offsets, offsets, (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_offsets, offsets, (n + 1) * sizeof(int32_t)));
   if (total) {
-    CK(cudaMemcpy(c->d_px, px, total * sizeof(int32_t), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->d_py, py, total * sizeof(int32_t), cudaMemcpyHostToDevice));
+    CK(upload(c, c->d_px, px, total * sizeof(int32_t)));
+    CK(upload(c, c->d_py, py, total * sizeof(int32_t)));
   }
   c->use_lists = true;
   c->list_npix_max = 0;
@@ -855,7 +864,7 @@ static int upload_force(dicegpu_ctx* c) {
   cudaStreamSynchronize(c->stream);
   int rc = grow(&c->d_force, &c->force_cap, (size_t)n);
   if (rc) return rc;
-  CK(cudaMemcpy(c->d_force, f.data(), n, cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_force, f.data(), n));
   c->use_force = true;
   return DICEGPU_OK;
 }
@@ -958,13 +967,13 @@ extern "C" int dicegpu_set_subset_shapes(dicegpu_ctx* c, int n_shapes, const dic
                 c->d_fields, c->params.subset_size >= 1 ? c->params.subset_size / 2 : -1,
                 any_evo ? 1 : 0, nullptr, any_evo ? c->d_evo_nact0.p : nullptr};
   const unsigned blocks = (unsigned)std::min<int64_t>(((int64_t)n * 32 + 255) / 256, (int64_t)c->num_sms * 8);
-  cudaError_t e = cudaMemcpy(c->d_shapes.p, grouped.data(), n_shapes * sizeof(dicegpu_shape), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_shape_off.p, shape_off.data(), (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice);
+  cudaError_t e = upload(c, c->d_shapes.p, grouped.data(), n_shapes * sizeof(dicegpu_shape));
+  if (e == cudaSuccess) e = upload(c, c->d_shape_off.p, shape_off.data(), (n + 1) * sizeof(int32_t));
   if (e == cudaSuccess && n_vertices) {
-    e = cudaMemcpy(c->d_svx.p, vx, n_vertices * sizeof(int32_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_svy.p, vy, n_vertices * sizeof(int32_t), cudaMemcpyHostToDevice);
+    e = upload(c, c->d_svx.p, vx, n_vertices * sizeof(int32_t));
+    if (e == cudaSuccess) e = upload(c, c->d_svy.p, vy, n_vertices * sizeof(int32_t));
   }
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_conformal.p, conformal.data(), n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(c, c->d_conformal.p, conformal.data(), n);
   if (e == cudaSuccess) {
     raster_kernel<false><<<blocks, 256, 0, c->stream>>>(ra);
     ++c->launches;
@@ -986,7 +995,7 @@ extern "C" int dicegpu_set_subset_shapes(dicegpu_ctx* c, int n_shapes, const dic
   size_t cap2 = c->list_cap;
   if ((rc = grow(&c->d_px, &c->list_cap, total)) || (rc = grow(&c->d_py, &cap2, total))) return rc;
   c->list_cap = std::min(c->list_cap, cap2);
-  CK(cudaMemcpy(c->d_offsets, offsets.data(), (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_offsets, offsets.data(), (n + 1) * sizeof(int32_t)));
   if (any_evo) {
     const size_t t1 = std::max<size_t>(total, 1);
     if ((rc = c->d_pix_flag0.ensure(t1)) || (rc = c->d_pix_flag.ensure(t1)) || (rc = c->d_pix_f.ensure(t1)))
@@ -1075,8 +1084,7 @@ extern "C" int dicegpu_set_blocking(dicegpu_ctx* c, const int32_t* offsets, cons
       }
       // the device descriptors exist once an obstruction or a tracking frame needed them
       if (c->d_mask_desc.p && c->d_mask_desc.cap >= c->h_mask_desc.size())
-        CK(cudaMemcpy(c->d_mask_desc.p, c->h_mask_desc.data(), c->h_mask_desc.size() * sizeof(int32_t),
-                      cudaMemcpyHostToDevice));
+        CK(upload(c, c->d_mask_desc.p, c->h_mask_desc.data(), c->h_mask_desc.size() * sizeof(int32_t)));
       c->use_masks = any;
       c->blocking_desc_ready = false;
     }
@@ -1127,10 +1135,10 @@ extern "C" int dicegpu_set_blocking(dicegpu_ctx* c, const int32_t* offsets, cons
       (rc = c->d_bpoly.ensure(6 * (size_t)std::max<int64_t>(dp_total, 1))) ||
       (rc = c->d_snapshot.ensure((size_t)n * DICEGPU_FIELD_STRIDE)))
     return rc;
-  CK(cudaMemcpy(c->d_blk_off.p, offsets, (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice));
-  if (offsets[n]) CK(cudaMemcpy(c->d_blk_ids.p, ids, offsets[n] * sizeof(int32_t), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_dv_off.p, dv_off.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_dp_off.p, dp_off.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_blk_off.p, offsets, (n + 1) * sizeof(int32_t)));
+  if (offsets[n]) CK(upload(c, c->d_blk_ids.p, ids, offsets[n] * sizeof(int32_t)));
+  CK(upload(c, c->d_dv_off.p, dv_off.data(), n * sizeof(int32_t)));
+  CK(upload(c, c->d_dp_off.p, dp_off.data(), n * sizeof(int32_t)));
   c->h_blk_off.assign(offsets, offsets + n + 1);
   c->h_blk_ids.assign(ids, ids + offsets[n]);
   c->h_has_polys.swap(has_polys);
@@ -1154,8 +1162,7 @@ static int ensure_blocking_desc(dicegpu_ctx* c) {
     int32_t* d = &c->h_mask_desc[(size_t)i * DG_MASK_DESC];
     d[5] = d[6] = 0;
   }
-  CK(cudaMemcpy(c->d_mask_desc.p, c->h_mask_desc.data(), c->h_mask_desc.size() * sizeof(int32_t),
-                cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_mask_desc.p, c->h_mask_desc.data(), c->h_mask_desc.size() * sizeof(int32_t)));
   c->blocking_desc_ready = true;
   c->use_masks = true;
   return DICEGPU_OK;
@@ -1214,9 +1221,9 @@ static int build_vsg_grid(dicegpu_ctx* c, int window) {
     }
   }
   if ((rc = c->d_vsg_cell_off.ensure(off.size()))) return rc;
-  CK(cudaMemcpy(c->d_vsg_cell_off.p, off.data(), off.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_vsg_cell_pts.p, pts.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_vsg_pos.p, pos.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_vsg_cell_off.p, off.data(), off.size() * sizeof(int32_t)));
+  CK(upload(c, c->d_vsg_cell_pts.p, pts.data(), n * sizeof(int32_t)));
+  CK(upload(c, c->d_vsg_pos.p, pos.data(), n * sizeof(int32_t)));
   c->h_vsg_coords.swap(coords);
   c->vsg_ncx = ncx;
   c->vsg_ncy = ncy;
@@ -1292,7 +1299,7 @@ static int build_vsg_knn(dicegpu_ctx* c, int k) {
   }
   int rc;
   if ((rc = c->d_vsg_nbr.ensure(nbr.size()))) return rc;
-  CK(cudaMemcpy(c->d_vsg_nbr.p, nbr.data(), nbr.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, c->d_vsg_nbr.p, nbr.data(), nbr.size() * sizeof(int32_t)));
   c->h_vsg_coords.resize(2 * (size_t)n);
   for (int i = 0; i < n; ++i) {
     c->h_vsg_coords[2 * i] = rows[(size_t)i * DICEGPU_FIELD_STRIDE + DICEGPU_F_COORD_X];
@@ -1659,9 +1666,9 @@ static int build_plan(dicegpu_ctx* c, int kind) {
   }
   int rc;
   if ((rc = pl.d_wave.ensure(n)) || (rc = pl.d_bwave.ensure(std::max<size_t>(bwave.size(), 1)))) return rc;
-  CK(cudaMemcpy(pl.d_wave.p, wave.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
+  CK(upload(c, pl.d_wave.p, wave.data(), n * sizeof(int32_t)));
   if (!bwave.empty())
-    CK(cudaMemcpy(pl.d_bwave.p, bwave.data(), bwave.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    CK(upload(c, pl.d_bwave.p, bwave.data(), bwave.size() * sizeof(int32_t)));
   pl.wave_off.swap(wave_off);
   pl.bwave_off.swap(bwave_off);
   pl.valid = true;
@@ -1937,9 +1944,9 @@ extern "C" int dicegpu_capture_sequence(dicegpu_ctx* c, int n, const float* cons
   if (incr && reset_fields) {
     const int rcs = c->d_ref_saved.ensure(3 * npx);
     if (rcs) return rcs;
-    CK(cudaMemcpy(c->d_ref_saved.p, c->d_ref, npx * sizeof(float), cudaMemcpyDeviceToDevice));
-    CK(cudaMemcpy(c->d_ref_saved.p + npx, c->d_ref_gx, npx * sizeof(float), cudaMemcpyDeviceToDevice));
-    CK(cudaMemcpy(c->d_ref_saved.p + 2 * npx, c->d_ref_gy, npx * sizeof(float), cudaMemcpyDeviceToDevice));
+    CK(cudaMemcpyAsync(c->d_ref_saved.p, c->d_ref, npx * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->d_ref_saved.p + npx, c->d_ref_gx, npx * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->d_ref_saved.p + 2 * npx, c->d_ref_gy, npx * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
   }
   if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
   if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
